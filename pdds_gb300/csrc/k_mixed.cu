@@ -37,7 +37,18 @@ struct ItemSide {
   int64_t map_off;
 };
 
+// Kinds whose Y changes along a path (a reaction term, or Robin local time).
+// For the others Y is 1 throughout, and the path carries no Y at all: the
+// products with it drop out with the same roundings.
+template <int KIND>
+constexpr bool has_y = KindTraits<KIND>::react || KIND == PK_ROBIN;
+
 constexpr unsigned FULL = 0xffffffffu;
+
+template <bool B>
+struct BoolC {
+  static constexpr bool value = B;
+};
 
 // State of one level of a path.  With table-served coefficients the level
 // also carries the 8 table fields at its position: the end-of-step sample
@@ -57,11 +68,19 @@ template <>
 struct Lvl<PK_LUT_TEX> : Lvl<PK_LUT> {};
 
 // Exit queue of a warp: a lane whose path pair has finished pushes both
-// levels' exit states (x, y, Y, Z + xi of the fine level, then of the coarse
-// level, then the step-limit flags) and the warp processes 32 pairs at a
-// time, one per lane.  <= 31 left over + one push of 32; slot XQCAP is the
-// spare slot written by lanes that push nothing.
+// levels' exit states (x, y, Z + xi and, where it varies, Y; the fine level,
+// then the coarse one) as pairs of words, and the warp processes 32 pairs at
+// a time, one per lane.  <= 31 left over + one push of 32; slot XQCAP is the
+// spare slot written by lanes that push nothing.  After the queue, one word
+// per slot holds the step-limit flags: written and read only once the warp
+// has come near the step limit.
 constexpr int XQCAP = 64;
+constexpr int queue_pairs(bool rich, bool y) { return ((y ? 4 : 3) * (rich ? 2 : 1) + 1) / 2; }
+// words of a warp's queue and flags: even, so that every warp's pairs are
+// 8-byte aligned
+constexpr int queue_words(bool rich, bool y) { return 2 * queue_pairs(rich, y) * (XQCAP + 1) + XQCAP + 2; }
+static_assert(queue_words(true, true) % 2 == 0 && queue_words(true, false) % 2 == 0 &&
+              queue_words(false, true) % 2 == 0 && queue_words(false, false) % 2 == 0, "pairs are 8-byte aligned");
 
 // Kahan step: s + c tracks the exact sum to O(eps^2); c holds the negated
 // rounding error of the running sum.
@@ -87,16 +106,33 @@ __device__ __forceinline__ float2 normals_f32(uint32_t ua, uint32_t ub) {
 }
 
 // path_block (counter = (step pair, path, knot, instance)) with the key
-// schedule read from the kernel parameters: the same stream.
-__device__ __forceinline__ u32x4 path_block_rk(const uint32_t (&rk)[20], uint32_t instance, uint32_t knot,
-                                               uint32_t path, uint32_t step_pair) {
+// schedule read from the kernel parameters: the same stream.  Of the first
+// two rounds, what depends on the knot alone (philox_knot) is formed once per
+// work item and what depends on the path once per path (philox_path); a block
+// then takes 17 multiplies instead of 20.
+struct PhiloxKnot {
+  uint32_t hi1, lo1;  // M1 * knot
+};
+struct PhiloxPath {
+  uint32_t a, b;  // round 2's words 2 (without the step pair's part) and 3
+};
+__device__ __forceinline__ PhiloxKnot philox_knot(uint32_t knot) {
+  return {__umulhi(0xCD9E8D57u, knot), 0xCD9E8D57u * knot};
+}
+__device__ __forceinline__ PhiloxPath philox_path(const uint32_t (&rk)[20], const PhiloxKnot& k, uint32_t path) {
+  const uint32_t v0 = k.hi1 ^ path ^ rk[0];
+  return {__umulhi(0xD2511F53u, v0) ^ rk[3], 0xD2511F53u * v0};
+}
+__device__ __forceinline__ u32x4 philox_block(const uint32_t (&rk)[20], uint32_t instance, const PhiloxKnot& k,
+                                              const PhiloxPath& p, uint32_t step_pair) {
+  const uint32_t v2 = __umulhi(0xD2511F53u, step_pair) ^ instance ^ rk[1];
   u32x4 c;
-  c.v[0] = step_pair;
-  c.v[1] = path;
-  c.v[2] = knot;
-  c.v[3] = instance;
+  c.v[0] = __umulhi(0xCD9E8D57u, v2) ^ k.lo1 ^ rk[2];
+  c.v[1] = 0xCD9E8D57u * v2;
+  c.v[2] = p.a ^ (0xD2511F53u * step_pair);
+  c.v[3] = p.b;
 #pragma unroll
-  for (int r = 0; r < 10; ++r) {
+  for (int r = 2; r < 10; ++r) {
     const uint32_t hi0 = __umulhi(0xD2511F53u, c.v[0]), lo0 = 0xD2511F53u * c.v[0];
     const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.v[2]), lo1 = 0xCD9E8D57u * c.v[2];
     u32x4 n;
@@ -107,6 +143,25 @@ __device__ __forceinline__ u32x4 path_block_rk(const uint32_t (&rk)[20], uint32_
     c = n;
   }
   return c;
+}
+__device__ __forceinline__ u32x4 path_block_rk(const uint32_t (&rk)[20], uint32_t instance, uint32_t knot,
+                                               uint32_t path, uint32_t step_pair) {
+  const PhiloxKnot k = philox_knot(knot);
+  return philox_block(rk, instance, k, philox_path(rk, k, path), step_pair);
+}
+
+// Smallest float a >= 0 for which a - hw < t fails (the rounded difference
+// is monotone in a, so a bisection over the bit patterns finds it): with
+// a(hw, t) formed once per item, the exit test |x - c| - hw < t of a step is
+// the single comparison |x - c| < a, with the same outcome for every x.
+__device__ __forceinline__ float exit_edge(float hw, float t) {
+  unsigned lo = 0u, hi = 0x7f800000u;
+  while (lo < hi) {
+    const unsigned mid = (lo + hi) >> 1;
+    if (__fsub_rn(__uint_as_float(mid), hw) < t) lo = mid + 1;
+    else hi = mid;
+  }
+  return __uint_as_float(lo);
 }
 
 // Table-served coefficients sampled from the nodes (PK_LUT) need more live
@@ -123,21 +178,24 @@ __global__ void __launch_bounds__(MIXED_MAX_THREADS, KIND == PK_LUT ? 2 : (KIND 
 k_paths_mixed(const MixedArgs a) {
   // dynamic shared memory: the warps' exit queues, then the exit histograms
   // [sum nbins] (and the Y^2 histogram after them)
-  extern __shared__ float dyn[];
+  extern __shared__ __align__(16) float dyn[];
   __shared__ ItemSide s_side[4];
   __shared__ float s_rect[4];
   __shared__ float s_dir[4];  // polar stencils: (cos, sin) of phi0 and phi1
   __shared__ int s_item, s_knot, s_p0, s_path_end, s_hist_len;
   __shared__ float s_h, s_sqrth;
+  __shared__ float s_edge[4];  // exit edges: fine x, fine y, coarse x, coarse y
   __shared__ unsigned s_next_path;
   __shared__ double s_red[MIXED_MAX_THREADS / 32][4];
   __shared__ unsigned long long s_redi[MIXED_MAX_THREADS / 32][3];
   __shared__ unsigned s_sth[32];  // this item's paths by steps (log2 bins), when step_hist is set
   __shared__ double s_dg[DIAG ? PDDS_DIAG_N : 1];  // this item's diagnostic sums (DIAG)
-  // exit queue of each warp: word w of slot i at q[w][i]
-  constexpr int QW = RICH ? 9 : 5;
+  constexpr bool HASY = has_y<KIND>;
+  // constant sigma on a rectangle: the exit test is two comparisons
+  constexpr bool EDGES = KindTraits<KIND>::iso && KIND != PK_ROBIN && GEOM == 0;
+  constexpr int QP = queue_pairs(RICH, HASY), QW = queue_words(RICH, HASY);
   const int nthr = blockDim.x, nwarps = nthr >> 5;
-  float* hist = dyn + nwarps * QW * (XQCAP + 1);
+  float* hist = dyn + nwarps * QW;
   const DevLayout& L = a.L;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -235,6 +293,16 @@ k_paths_mixed(const MixedArgs a) {
     if (tid < 32) s_sth[tid] = 0u;
     if (DIAG && tid < PDDS_DIAG_N) s_dg[tid] = 0.0;
     float* hist2 = hist + hist_len;
+    // increment scales (sqrt2 sqrt(h) for iso kinds, sqrt(h) otherwise) and
+    // Gobet thresholds of the fine (h/2) and coarse (h) levels
+    const float hf = 0.5f * h;
+    const float scc = KindTraits<KIND>::iso ? 1.41421356f * sqrth : sqrth;
+    const float scf = scc * 0.70710678f;
+    const float thrc = -0.5826f * scc, thrf = -0.5826f * scf;
+    if (EDGES && tid < 4) {
+      const float lo = s_rect[tid & 1], up = s_rect[2 + (tid & 1)];
+      s_edge[tid] = exit_edge(up - 0.5f * (lo + up), tid < 2 && RICH ? thrf : thrc);
+    }
     __syncthreads();
 
     // ------------------------------------------------------------ paths
@@ -290,15 +358,12 @@ k_paths_mixed(const MixedArgs a) {
     unsigned nglob = 0, nsten = 0;  // exits of the lane in this item (<= 2 N)
     int qcount = 0;  // warp-uniform
     const unsigned lt = (1u << lane) - 1u;
-    float (*q)[XQCAP + 1] = reinterpret_cast<float (*)[XQCAP + 1]>(dyn + warp * QW * (XQCAP + 1));
+    // word pair w of slot i at q2[w][i], its step-limit flags at qmeta[i]
+    float2 (*q2)[XQCAP + 1] = reinterpret_cast<float2 (*)[XQCAP + 1]>(dyn + warp * QW);
+    unsigned* qmeta = reinterpret_cast<unsigned*>(q2 + QP);
     const bool use_cv = P.use_cv != 0;
-    // increment scales (sqrt2 sqrt(h) for iso kinds, sqrt(h) otherwise) and
-    // Gobet thresholds of the fine (h/2) and coarse (h) levels
-    const float hf = 0.5f * h;
-    const float scc = KindTraits<KIND>::iso ? 1.41421356f * sqrth : sqrth;
-    const float scf = scc * 0.70710678f;
-    const float thrc = -0.5826f * scc, thrf = -0.5826f * scf;
     const unsigned maxs = (unsigned)a.max_steps;
+    const float2 edge_f = make_float2(s_edge[0], s_edge[1]), edge_c = make_float2(s_edge[2], s_edge[3]);
 
     // One step of a level (Step, control-variate variant,
     // FKACIntegrator.hpp:46-57) and the Gobet-shifted exit test (Inside,
@@ -321,7 +386,10 @@ k_paths_mixed(const MixedArgs a) {
     // The (x, y) arithmetic of a step runs as paired FP32 instructions
     // (FADD2 / FMUL2 / FFMA2: two lanes' worth of work per issue slot, the
     // same roundings as the scalar pair).
-    auto advance = [&](Lvl<KIND>& s, float2 e, float hh, float thr, float ex) -> bool {
+    // `limit`: the step counts as an exit when the level has reached the step
+    // limit (only rounds near it test that).
+    auto advance = [&](Lvl<KIND>& s, float2 e, float hh, float thr, float2 edge, float ex, auto limit) -> bool {
+      const auto at_limit = [&]() -> bool { return decltype(limit)::value && s.steps >= maxs; };
       Coef<float> k;
       if constexpr (is_lut_kind(KIND)) {
         k.s00 = s.cf[0]; k.s11 = s.cf[1];
@@ -333,8 +401,13 @@ k_paths_mixed(const MixedArgs a) {
       float2 d = e;
       if constexpr (!KindTraits<KIND>::iso) d = __fmul2_rn(make_float2(k.s00, k.s11), e);
       const float d0 = d.x, d1 = d.y;
-      s.xi -= s.Y * (k.g0 * d0 + k.g1 * d1);
-      s.Z += k.f * s.Y * hh;
+      if constexpr (HASY) {
+        s.xi -= s.Y * (k.g0 * d0 + k.g1 * d1);
+        s.Z += k.f * s.Y * hh;
+      } else {
+        s.xi = __fsub_rn(s.xi, k.g0 * d0 + k.g1 * d1);
+        s.Z = fmaf(k.f, hh, s.Z);
+      }
       if constexpr (KindTraits<KIND>::react) s.Y += k.c * s.Y * hh;
       if constexpr (KIND == PK_ROBIN) {
         float dL = 0.f;
@@ -359,7 +432,7 @@ k_paths_mixed(const MixedArgs a) {
         ++s.steps;
         float o[4];
         absorb_out(s.x, s.y, o);
-        return !(fmaxf(fmaxf(o[0], o[1]), fmaxf(o[2], o[3])) < thr) || s.steps >= (unsigned)a.max_steps;
+        return !(fmaxf(fmaxf(o[0], o[1]), fmaxf(o[2], o[3])) < thr) || at_limit();
       } else if constexpr (KindTraits<KIND>::iso) {
         const float2 np = __fadd2_rn(make_float2(s.x, s.y), d);
         s.x = np.x;
@@ -375,7 +448,10 @@ k_paths_mixed(const MixedArgs a) {
         float d_in, d_out, d_a, d_b;
         polar_out(s.x, s.y, d_in, d_out, d_a, d_b);
         const float dist = fmaxf(fmaxf(d_in, d_out), fmaxf(d_a, d_b));
-        return !(dist < thr) || s.steps >= (unsigned)a.max_steps;
+        return !(dist < thr) || at_limit();
+      } else if constexpr (EDGES) {
+        const float2 o = __fadd2_rn(make_float2(s.x, s.y), make_float2(-cx, -cy));
+        return !(fabsf(o.x) < edge.x) || !(fabsf(o.y) < edge.y) || at_limit();
       } else {
         const float dx = fabsf(s.x - cx) - hx, dy = fabsf(s.y - cy) - hy;
         float t = thr;
@@ -387,7 +463,7 @@ k_paths_mixed(const MixedArgs a) {
           sigma_normals_f32<KIND>(P, s.x, s.y, nx, ny);
           t *= dx > dy ? nx : ny;
         }
-        return !(fmaxf(dx, dy) < t) || s.steps >= (unsigned)a.max_steps;
+        return !(fmaxf(dx, dy) < t) || at_limit();
       }
     };
     // Value of one exit of a level, weighted: projection onto the stencil
@@ -457,7 +533,8 @@ k_paths_mixed(const MixedArgs a) {
             glob = true;
             float sa, ca;
             sincosf(ang, &sa, &ca);
-            val += Y * u_f32<KIND>(P, rect[2] * ca, rect[2] * sa);
+            const float g = u_f32<KIND>(P, rect[2] * ca, rect[2] * sa);
+            val = HASY ? fmaf(Y, g, val) : __fadd_rn(val, g);
           }
         } else {
           const float t = d == 3 ? ua0 * x + ua1 * y : ub0 * x + ub1 * y;
@@ -517,7 +594,8 @@ k_paths_mixed(const MixedArgs a) {
         }
         if (onmask & globmask) {
           ++nglob;
-          val += Y * u_f32<KIND>(P, Ex, Ey);
+          const float g = u_f32<KIND>(P, Ex, Ey);
+          val = HASY ? fmaf(Y, g, val) : __fadd_rn(val, g);
         } else {
           ++nsten;
           const ItemSide& is = s_side[d];
@@ -549,41 +627,46 @@ k_paths_mixed(const MixedArgs a) {
     };
     Lvl<KIND> F, Cs;  // fine (or only) and coarse level of the lane's pair
     // Push the finished pairs of the warp (both levels' exit states; the
-    // warp-synchronous ballot gives each its slot) and return their mask.
-    // Lanes without a finished pair write the spare slot XQCAP instead of
-    // branching around the stores.
-    auto push = [&](bool ex) -> unsigned {
-      const unsigned mk = __ballot_sync(FULL, ex);
+    // warp-synchronous ballot gives each its slot).  Lanes without a finished
+    // pair write the spare slot XQCAP instead of branching around the stores.
+    // A level's words: x, y, value (and Y): two pairs with Y, otherwise the
+    // levels' values share a pair.
+    // table-served kinds: one round between two looks, which tests the limit
+    constexpr bool SINGLE = is_lut_kind(KIND);
+    bool near_limit = SINGLE;  // warp-uniform: a round of this item has tested the step limit
+    auto push = [&](bool ex, unsigned mk) {
       int i = ex ? qcount + __popc(mk & lt) : XQCAP;
       if (!idx_ok(i, XQCAP + 1, a.err_flags)) i = XQCAP;
-      q[0][i] = F.x;
-      q[1][i] = F.y;
-      q[2][i] = F.Y;
-      q[3][i] = use_cv ? F.Z + F.xi : F.Z;
-      unsigned meta = F.steps >= maxs ? 1u : 0u;
-      if (RICH) {
-        q[4][i] = Cs.x;
-        q[5][i] = Cs.y;
-        q[6][i] = Cs.Y;
-        q[7][i] = use_cv ? Cs.Z + Cs.xi : Cs.Z;
-        meta |= Cs.steps >= maxs ? 2u : 0u;
+      const float vf = use_cv ? F.Z + F.xi : F.Z;
+      const float vc = RICH ? (use_cv ? Cs.Z + Cs.xi : Cs.Z) : 0.f;
+      q2[0][i] = make_float2(F.x, F.y);
+      if constexpr (HASY) {
+        q2[1][i] = make_float2(vf, F.Y);
+        if constexpr (RICH) {
+          q2[2][i] = make_float2(Cs.x, Cs.y);
+          q2[3][i] = make_float2(vc, Cs.Y);
+        }
+      } else {
+        q2[1][i] = make_float2(vf, vc);
+        if constexpr (RICH) q2[2][i] = make_float2(Cs.x, Cs.y);
       }
-      q[QW - 1][i] = __uint_as_float(meta);
+      if (near_limit) qmeta[i] = (F.steps >= maxs ? 1u : 0u) | (RICH && Cs.steps >= maxs ? 2u : 0u);
       qcount += __popc(mk);
-      return mk;
     };
     // Process the pair at queue index i (lane-parallel): both exits scored,
     // B += 2 v_fine - v_coarse (v otherwise) in the lane's compensated sums.
     auto process = [&](int i, bool valid) {
       if (valid) {
-        const unsigned meta = __float_as_uint(q[QW - 1][i]);
+        const unsigned meta = near_limit ? qmeta[i] : 0u;
         float v = 0.f;
 #pragma unroll 1
         for (int lv = 0; lv < (RICH ? 2 : 1); lv++) {
-          const int o = 4 * lv;
           const float wgt = RICH ? (lv ? -1.f : 2.f) : 1.f;
           const float sql = (RICH && lv == 0) ? sqrth * 0.70710678f : sqrth;
-          v += score(q[o][i], q[o + 1][i], q[o + 2][i], q[o + 3][i], wgt, ((meta >> lv) & 1u) != 0, sql);
+          const float2 xy = q2[2 * lv][i];
+          const float2 vy = q2[HASY ? 2 * lv + 1 : 1][i];
+          const float val = HASY ? vy.x : (lv ? vy.y : vy.x), Y = HASY ? vy.y : 1.f;
+          v += score(xy.x, xy.y, Y, val, wgt, ((meta >> lv) & 1u) != 0, sql);
         }
         kahan_add(bs, bc, v);
         kahan_add(bbs, bbc, v * v);
@@ -608,6 +691,8 @@ k_paths_mixed(const MixedArgs a) {
 
     float cf0[8];  // table fields at the knot (table-served kinds)
     if constexpr (is_lut_kind(KIND)) lut_sample_f32<KIND, 8>(P.lut, x0, y0, cf0);
+    const PhiloxKnot pk = philox_knot(rng_knot);
+    PhiloxPath pp;
     auto reset = [&]() {
       F.x = x0; F.y = y0; F.Y = 1.f; F.Z = 0.f; F.xi = 0.f; F.steps = 0;
       if constexpr (is_lut_kind(KIND)) {
@@ -615,56 +700,95 @@ k_paths_mixed(const MixedArgs a) {
         for (int f = 0; f < 8; f++) F.cf[f] = cf0[f];
       }
       Cs = F;
+      pp = philox_path(a.rk, pk, path);
     };
     reset();
     bool f_alive = active, c_alive = RICH && active;
     unsigned m = 0;
-    while (__any_sync(FULL, active)) {
-      if (active) {
-        const unsigned mi = m++;
-        const u32x4 blk = path_block_rk(a.rk, rng_inst, rng_knot, path, mi);
-        const float2 za = normals_f32(blk.v[0], blk.v[1]), zb = normals_f32(blk.v[2], blk.v[3]);
-        // Exp(1) samples of the reflected steps: a second Philox block with
-        // the knot word's top bit set (fine A, fine B, coarse)
-        float x0e = 0.f, x1e = 0.f, x2e = 0.f;
-        if (KIND == PK_ROBIN && rmask) {
-          const u32x4 bx = path_block_rk(a.rk, rng_inst, rng_knot | 0x80000000u, path, mi);
-          x0e = -0.69314718f * lg2_approx(fmaf((float)bx.v[0], 2.3283064e-10f, 1.1641532e-10f));
-          x1e = -0.69314718f * lg2_approx(fmaf((float)bx.v[1], 2.3283064e-10f, 1.1641532e-10f));
-          x2e = -0.69314718f * lg2_approx(fmaf((float)bx.v[2], 2.3283064e-10f, 1.1641532e-10f));
-        }
-        if (RICH) {
-          // Richardson pair: two fine steps of h/2 and one coarse step of h
-          // on the same Brownian increments (dW_coarse = dW_fine1 + dW_fine2);
-          // 2 E[fine] - E[coarse] cancels the O(h) bias.  A level that has
-          // exited keeps its exit state until the pair is pushed.
-          const float2 sf = make_float2(scf, scf);
-          const float2 ea = __fmul2_rn(sf, za), eb = __fmul2_rn(sf, zb);
-          if (f_alive) {
-            bool fx = advance(F, ea, hf, thrf, x0e);
-            if (!fx) fx = advance(F, eb, hf, thrf, x1e);
-            f_alive = !fx;
-          }
-          if (c_alive) c_alive = !advance(Cs, __fadd2_rn(ea, eb), h, thrc, x2e);
-        } else {
-          const float2 sc = make_float2(scc, scc);
-          bool fx = advance(F, __fmul2_rn(sc, za), h, thrc, x0e);
-          if (!fx) fx = advance(F, __fmul2_rn(sc, zb), h, thrc, x1e);
+    // One round of the lane's pair: one Philox block and its level steps.
+    auto round = [&](auto limit) {
+      const unsigned mi = m++;
+      const u32x4 blk = philox_block(a.rk, rng_inst, pk, pp, mi);
+      const float2 za = normals_f32(blk.v[0], blk.v[1]), zb = normals_f32(blk.v[2], blk.v[3]);
+      // Exp(1) samples of the reflected steps: a second Philox block with
+      // the knot word's top bit set (fine A, fine B, coarse)
+      float x0e = 0.f, x1e = 0.f, x2e = 0.f;
+      if (KIND == PK_ROBIN && rmask) {
+        const u32x4 bx = path_block_rk(a.rk, rng_inst, rng_knot | 0x80000000u, path, mi);
+        x0e = -0.69314718f * lg2_approx(fmaf((float)bx.v[0], 2.3283064e-10f, 1.1641532e-10f));
+        x1e = -0.69314718f * lg2_approx(fmaf((float)bx.v[1], 2.3283064e-10f, 1.1641532e-10f));
+        x2e = -0.69314718f * lg2_approx(fmaf((float)bx.v[2], 2.3283064e-10f, 1.1641532e-10f));
+      }
+      if (RICH) {
+        // Richardson pair: two fine steps of h/2 and one coarse step of h
+        // on the same Brownian increments (dW_coarse = dW_fine1 + dW_fine2);
+        // 2 E[fine] - E[coarse] cancels the O(h) bias.  A level that has
+        // exited keeps its exit state until the pair is pushed.
+        const float2 sf = make_float2(scf, scf);
+        const float2 ea = __fmul2_rn(sf, za), eb = __fmul2_rn(sf, zb);
+        if (f_alive) {
+          bool fx = advance(F, ea, hf, thrf, edge_f, x0e, limit);
+          if (!fx) fx = advance(F, eb, hf, thrf, edge_f, x1e, limit);
           f_alive = !fx;
         }
+        if (c_alive) c_alive = !advance(Cs, __fadd2_rn(ea, eb), h, thrc, edge_c, x2e, limit);
+      } else {
+        const float2 sc = make_float2(scc, scc);
+        bool fx = advance(F, __fmul2_rn(sc, za), h, thrc, edge_c, x0e, limit);
+        if (!fx) fx = advance(F, __fmul2_rn(sc, zb), h, thrc, edge_c, x1e, limit);
+        f_alive = !fx;
       }
+    };
+    // Rounds run in groups between two looks for finished pairs (queueing
+    // their exits and refilling their lanes).  A look costs about a third of
+    // a round in instructions, a lane that finishes early in a group idles to
+    // its end: with p the share of lanes that finish per round, the cost
+    // 1 / g + (p / 2)(g - 1) per round is least at g ~ sqrt(GAP / (32 p)),
+    // and p is what this warp has counted in this item so far.  Path kernel,
+    // against a look after every round (and Y, per-step limit tests and the
+    // four-operation exit test, which went at the same time): 12x12/n43
+    // 27.3 -> 25.0 ms, the circle at h = 2e-5 (270 rounds per pair) 341 ->
+    // 290 ms; GAP 8, 14, 22, 32 and 36 measured 27.4, 26.7, 25.2, 25.0 and
+    // 25.0 ms on the former.  A round of
+    // the table-served kinds is bound by its table reads, which idle lanes
+    // do not shorten (groups measured 1-2 % slower there): they look after
+    // every round.
+    constexpr float GAP = RICH ? 32.f : 48.f;
+    constexpr int GAP_MAX = 32;
+    unsigned rounds = 0, found = 0;  // warp-uniform
+    int gap = SINGLE ? 1 : 2;
+    const unsigned far = maxs > 0 ? (maxs - 1) / 2 : 0;  // rounds that cannot reach the step limit
+    while (__any_sync(FULL, active)) {
+      if constexpr (SINGLE) {
+        if (f_alive || c_alive) round(BoolC<true>{});
+      } else if (rounds + gap > far && __any_sync(FULL, active && m + gap > far)) {
+        if (!near_limit) {  // from here on pushes write the flags; none is set so far
+          near_limit = true;
+          qmeta[lane] = 0u;
+          qmeta[lane + 32] = 0u;
+          __syncwarp();
+        }
+        gap = 1;
+        if (f_alive || c_alive) round(BoolC<true>{});
+      } else {
+        for (int g = 0; g < gap; ++g)
+          if (f_alive || c_alive) round(BoolC<false>{});
+      }
+      rounds += gap;
       // finished pairs: queue both exits, then refill from the item's
       // path counter with one warp-aggregated atomic
       const bool done = active && !f_alive && !c_alive;
-      const unsigned dm = push(done);
-      drain_full();
+      const unsigned dm = __ballot_sync(FULL, done);
       if (dm) {
+        push(done, dm);
+        drain_full();
+        found += __popc(dm);
         const int leader = __ffs(dm) - 1;
         unsigned base = 0;
         if (lane == leader) base = atomicAdd(&s_next_path, (unsigned)__popc(dm));
         base = __shfl_sync(FULL, base, leader);
         if (done) {
-          if (a.step_hist) {  // finished pairs only: a few lanes per iteration
+          if (a.step_hist) {  // finished pairs only: a few lanes per look
             atomicAdd(&s_sth[31 - __clz(max(F.steps, 1u))], 1u);
             if (RICH) atomicAdd(&s_sth[31 - __clz(max(Cs.steps, 1u))], 1u);
           }
@@ -675,7 +799,7 @@ k_paths_mixed(const MixedArgs a) {
               float Ex, Ey, Nx, Ny;
               int om;
               rect2d<float>(rect, v.x, v.y, Ex, Ey, Nx, Ny, om);
-              return v.Z + v.Y * u_f32<KIND>(P, Ex, Ey);
+              return v.Z + (HASY ? v.Y : 1.f) * u_f32<KIND>(P, Ex, Ey);
             };
             float ph = phi_of(F), xv = F.xi;
             if (RICH) {
@@ -693,6 +817,8 @@ k_paths_mixed(const MixedArgs a) {
           m = 0;
         }
       }
+      if constexpr (!SINGLE)
+        gap = max(1, min(GAP_MAX, (int)sqrt_approx(__fdividef(GAP * (float)rounds, (float)(found + 1u)))));
     }
     drain_all();
     // ------------------------------------------------------------ reduce B
@@ -844,8 +970,8 @@ static bool is_mixed_t(const void* f) {
 
 bool is_mixed_path_kernel(const void* func) { return is_mixed_t<true>(func) || is_mixed_t<false>(func); }
 
-size_t mixed_queue_smem(int threads, int richardson) {
-  return (size_t)(threads / 32) * (richardson ? 9 : 5) * (XQCAP + 1) * sizeof(float);
+size_t mixed_queue_smem(int threads, int richardson) {  // with Y: the larger of the two forms
+  return (size_t)(threads / 32) * queue_words(richardson != 0, true) * sizeof(float);
 }
 
 cudaError_t launch_paths_mixed(const MixedArgs& a, int kind, int grid, int threads, size_t smem, cudaStream_t s) {
