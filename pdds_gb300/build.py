@@ -30,6 +30,7 @@ UNITS = {
     "k_misc.cu": ["-fmad=false"],
     "k_solve.cu": [],
     "k_gmres_cluster.cu": [],
+    "k_resident.cu": [],
     "batch.cu": [],
     "k_subdomain.cu": [],
     "layout.cpp": ["-x", "cu"],

@@ -265,6 +265,7 @@ pdds_status upload_layout(pdds_ctx* ctx) {
   ctx->has_solution = false;
   ctx->ugrid_m = 0;
   ctx->lpt_ready = false;
+  ctx->solve_plan[0].ready = ctx->solve_plan[1].ready = false;
   HostLayout& L = ctx->L;
   cudaStream_t s = ctx->stream;
   std::vector<double> st_rect;
@@ -828,6 +829,7 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     ctx->st_cols.recycle();
     ctx->map_owner.recycle();
     ctx->lay_block.recycle();
+    ctx->sexch.recycle();
     ctx->knot_rng.recycle();
     ctx->tab.recycle();
     ctx->lut_coef.recycle();
@@ -1772,8 +1774,55 @@ pdds_status pdds_solve_interface(pdds_ctx* ctx, const pdds_solve_desc* desc, dou
   int iters = 0, refines = 0;
   double relres = 0.0;
   const double tol = desc->tol > 0 ? desc->tol : 1e-10;
+  // the system resident on chip where it fits (its columns are the stencils'
+  // lists, which every layout has); the GMRES form with two barriers per step
+  // and larger systems run the kernels that read the matrix from L2
+  const bool bicg = desc->method == PDDS_SOLVE_BICGSTAB_FP64;
+  const int rmeth = bicg ? RESIDENT_BICGSTAB : RESIDENT_GMRES;
+  ResidentPlan plan;
+  if (!ctx->is_batch && (bicg || (desc->method == PDDS_SOLVE_GMRES_FP32_IR &&
+                                  desc->gmres_form == PDDS_GMRES_PIPELINED))) {
+    pdds_ctx::SolvePlan& sp = ctx->solve_plan[rmeth];
+    if (!sp.ready || sp.m != m || sp.grid_ctas != desc->grid_ctas) {
+      const ResidentRows rows{K, L.row_ptr.data(), L.knot_stencil.data()};
+      sp.plan = resident_plan(rows, rmeth, m, desc->grid_ctas);
+      sp.m = m;
+      sp.grid_ctas = desc->grid_ctas;
+      sp.ready = true;
+    }
+    plan = sp.plan;
+  }
   CK(cudaEventRecord(ctx->ev0, s));
-  if (desc->method == PDDS_SOLVE_BICGSTAB_FP64) {
+  if (plan.ctas > 0) {
+    CK(ctx->sexch.resize(resident_exchange_bytes(K)));
+    ResidentArgs a{};
+    a.K = K;
+    a.row_ptr = ctx->row_ptr.p;
+    a.knot_stencil = ctx->knot_stencil.p;
+    a.st_off = ctx->st_col_off.p;
+    a.st_cols = ctx->st_cols.p;
+    a.val64 = ctx->G.p;
+    a.b = ctx->B.p;
+    a.x = ctx->su.p;
+    a.m = m;
+    a.max_iter = desc->max_iter > 0 ? desc->max_iter : (bicg ? 2 * K : 1000);
+    a.max_refine = desc->max_refine > 0 ? desc->max_refine : 30;
+    a.tol = tol;
+    a.inner_tol = 1e-6;
+    a.out = ctx->sscal.p;
+    a.err_flags = ctx->errf.p;
+    a.spin_limit = w.spin_limit;
+    CK(launch_resident(a, plan, rmeth, ctx->sexch.p, s));
+    w.launches = 1;
+    double out[2] = {0.0, 0.0};
+    CK(copy_async(out, ctx->sscal.p, sizeof(out), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    int cnt[2];
+    std::memcpy(cnt, &out[1], sizeof(cnt));
+    relres = out[0];
+    iters = cnt[0];
+    refines = cnt[1];
+  } else if (desc->method == PDDS_SOLVE_BICGSTAB_FP64) {
     const int maxit = desc->max_iter > 0 ? desc->max_iter : 2 * K;
     CK(solve_bicgstab(A, ctx->B.p, ctx->su.p, w, maxit, tol, &iters, &relres, s));
   } else if (desc->method == PDDS_SOLVE_GMRES_FP32_IR) {

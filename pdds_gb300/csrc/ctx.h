@@ -11,6 +11,7 @@
 #include "../../include/pdds.h"
 #include "kernels.h"
 #include "pdds_internal.h"
+#include "solve.h"
 #include "xfer.h"
 
 namespace pdds {
@@ -162,7 +163,15 @@ struct pdds_ctx {
   DBuf<float> sV32, sw32, sval32, sZ32;
   DBuf<unsigned> sctl, sbar;
   DBuf<double> sgpart;
+  DBuf<unsigned char> sexch;  // words that the resident solve's CTAs exchange
   double* host_rr = nullptr;
+  // split of the system for the resident solve (RESIDENT_GMRES, RESIDENT_BICGSTAB),
+  // valid until the layout or these parameters change
+  struct SolvePlan {
+    bool ready = false;
+    int m = 0, grid_ctas = 0;
+    pdds::ResidentPlan plan;
+  } solve_plan[2];
   int solve_m = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   // batch of independent instances (pdds_batch_build): the layout above is

@@ -82,6 +82,54 @@ cudaError_t launch_stamp(unsigned long long* t, cudaStream_t s);
 // b[i] = (float)a[i]
 cudaError_t launch_to_f32(const double* a, float* b, int64_t n, cudaStream_t s);
 
+// One interface system with its rows resident on chip (k_resident.cu).
+// How the system is split: CTA c owns the rows [row0[c], row0[c + 1]), at
+// most `per`; cap_* are the largest CTA's entries (0: BiCGSTAB entries that stay in L2), column-list
+// entries (rows of one stencil share their list) and distinct columns, which
+// size its shared memory.
+constexpr int RESIDENT_MAX_CTAS = 160;
+struct ResidentPlan {
+  int ctas = 0;       // 0: the system does not fit
+  int row0[RESIDENT_MAX_CTAS + 1] = {0};
+  int per = 0;
+  int cap_nnz = 0, cap_list = 0, cap_loc = 0;
+  size_t smem = 0;
+};
+struct ResidentArgs {
+  int K;
+  const int64_t* row_ptr;
+  const int* knot_stencil;   // row k's columns are its stencil's list
+  const int64_t* st_off;
+  const int* st_cols;
+  const double* val64;
+  const double* b;
+  double* x;
+  int m, max_iter, max_refine;
+  double tol, inner_tol;
+  double* out;               // relative residual, then (iterations, refinements) as two ints
+  unsigned* err_flags;
+  unsigned spin_limit;       // polls before a wait gives up (0: the default, about a second)
+  // filled in by launch_resident
+  int row0[RESIDENT_MAX_CTAS + 1];
+  int per, cap_nnz, cap_list, cap_loc;
+  ulonglong2* part;          // tagged partials of the group sums
+  ulonglong2* pub;           // 2 K: tagged FP64 vectors (x; r and v)
+  unsigned long long* T;     // 2 K: tagged Krylov vectors
+};
+// Host rows of a layout: row k has row_ptr[k + 1] - row_ptr[k] entries, its
+// stencil's columns (none on the boundary).
+struct ResidentRows {
+  int K;
+  const int64_t* row_ptr;
+  const int32_t* knot_stencil;
+};
+enum { RESIDENT_GMRES = 0, RESIDENT_BICGSTAB = 1 };
+// The split of a system for `method` (m: the GMRES restart length); grid_ctas
+// > 0 bounds the number of CTAs.
+ResidentPlan resident_plan(const ResidentRows& rows, int method, int m, int grid_ctas);
+size_t resident_exchange_bytes(int K);  // device memory through which the CTAs exchange
+cudaError_t launch_resident(const ResidentArgs& a, const ResidentPlan& p, int method, void* exchange, cudaStream_t s);
+
 // The same solve through k_gmres_cluster for one system; *used is false (and
 // nothing ran) when the system does not fit the cluster kernel.
 cudaError_t solve_gmres_ir_cluster(const SolveCsr& A, const double* b, double* x, SolveWork& w, int m,
