@@ -819,10 +819,10 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     DBuf<int>* di[] = {&ctx->knot_stencil, &ctx->st_side, &ctx->st_glob, &ctx->map_pos, &ctx->sd_n,
                        &ctx->sd_orient, &ctx->sd_shape, &ctx->side_knot, &ctx->sh_n, &ctx->sh_nbins,
                        &ctx->col, &ctx->mc_knots, &ctx->bnd_knots, &ctx->counter, &ctx->rside,
-                       &ctx->rsl, &ctx->rss, &ctx->task_m, &ctx->task_d, &ctx->task_i, &ctx->rbf_piv};
+                       &ctx->rsl, &ctx->rss, &ctx->rbf_piv};
     for (auto* b : di) b->recycle();
     DBuf<int64_t>* dl[] = {&ctx->row_ptr, &ctx->st_map_off, &ctx->sd_knot_off, &ctx->sh_tab_off,
-                           &ctx->sh_ipsi_off, &ctx->sh_t_off, &ctx->task_out, &ctx->knot_task_off,
+                           &ctx->sh_ipsi_off, &ctx->sh_t_off, &ctx->knot_task_off,
                            &ctx->knot_ipsi_off};
     for (auto* b : dl) b->recycle();
     ctx->st_col_off.recycle();
@@ -1187,43 +1187,35 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
     if (diag) {
       DBuf<double>* db[] = {&ctx->rsx, &ctx->rsy, &ctx->rsY, &ctx->rsZ, &ctx->rsxi};
       for (auto* b : db) CK(b->resize(std::max<int64_t>(total, 1)));
-      CK(ctx->rknot_h.resize(std::max(rn, 1)));
     }
-    // (knot, side, side knot) tasks of the range's knots in hand-out order;
+    CK(ctx->rknot_h.resize(2 * std::max(rn, 1)));
+    // side entries of the range's knots in hand-out order;
     // knot m of the range is hand-out position r0 + m (ipsi_override packs
     // every knot, so its offsets count them all)
-    std::vector<int> tm, td, ti;
-    std::vector<int64_t> tout, ktoff(std::max(rn, 1), 0), kipoff(4 * std::max(rn, 1), -1);
-    std::vector<int> mc;
-    for (int v : L.order) if (!L.knot_boundary[v]) mc.push_back(v);
-    int64_t ipo = 0;
+    std::vector<int64_t> ktoff(std::max(rn, 1), 0), kipoff(4 * std::max(rn, 1), -1);
+    int64_t ipo = 0, nside = 0;
+    int max_n = 0;
     for (int mg = 0; mg < n_mc; mg++) {
-      const StencilRec& st = L.stencils[L.knot_stencil[mc[mg]]];
+      const StencilRec& st = L.stencils[L.knot_stencil[ctx->mc_host[mg]]];
       const bool in = mg >= r0 && mg < r0 + rn;
       const int m = mg - r0;
-      if (in) ktoff[m] = (int64_t)tm.size();
+      if (in) ktoff[m] = nside;
       for (int d = 0; d < 4; d++) {
         if (st.side[d] < 0) continue;
         const int n = L.sides[st.side[d]].n;
         if (in) kipoff[4 * m + d] = ipo;
         ipo += (int64_t)n * n;
         if (!in) continue;
-        for (int i = 0; i < n; i++) {
-          tm.push_back(m); td.push_back(d); ti.push_back(i);
-          tout.push_back((int64_t)tout.size());
-        }
+        nside += n;
+        max_n = std::max(max_n, n);
       }
     }
     if (desc->ipsi_override && desc->ipsi_override_len != ipo)
       return fail(ctx, PDDS_ERR_INVALID, "ipsi_override_len does not match the layout (expected " +
                                              std::to_string(ipo) + ")");
-    CK(ctx->task_m.upload(tm, s));
-    CK(ctx->task_d.upload(td, s));
-    CK(ctx->task_i.upload(ti, s));
-    CK(ctx->task_out.upload(tout, s));
     CK(ctx->knot_task_off.upload(ktoff, s));
-    CK(ctx->Gside.resize(std::max<size_t>(tm.size(), 1)));
-    CK(ctx->GGside.resize(std::max<size_t>(tm.size(), 1)));
+    CK(ctx->Gside.resize(std::max<int64_t>(nside, 1)));
+    CK(ctx->GGside.resize(std::max<int64_t>(nside, 1)));
     if (desc->ipsi_override) {
       CK(ctx->knot_ipsi_off.upload(kipoff, s));
       CK(ctx->ipsi_knot.resize(std::max<int64_t>(ipo, 1)));
@@ -1250,33 +1242,18 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
     a.diag = diag ? ctx->diag.p : nullptr;
     a.sx = diag ? ctx->rsx.p : nullptr; a.sy = diag ? ctx->rsy.p : nullptr;
     a.sY = diag ? ctx->rsY.p : nullptr; a.sZ = diag ? ctx->rsZ.p : nullptr;
-    a.sxi = diag ? ctx->rsxi.p : nullptr; a.knot_h = diag ? ctx->rknot_h.p : nullptr;
+    a.sxi = diag ? ctx->rsxi.p : nullptr; a.knot_h = ctx->rknot_h.p;
+    a.path_counter = ctx->stats.p + 7;
+    a.stats = ctx->stats.p;
     a.G = ctx->G.p;
     a.GG = ctx->GG.p;
     a.B = ctx->B.p;
     a.BB = ctx->BB.p;
     a.dup_sum = ctx->L.geom == 1 ? 1 : desc->dup_sum;  // circle layouts sum shared side knots
     a.err_flags = ctx->errf.p;
-    CK(launch_replay_paths(a, P.kind, s));
-    CK(launch_replay_reduce(a, P.kind, ctx->task_m.p, ctx->task_d.p, ctx->task_i.p, (int)tm.size(),
-                            ctx->task_out.p, ctx->knot_task_off.p, ctx->Gside.p, ctx->GGside.p, s));
-    launches += 4;
-    if (info) {
-      // step counts from the exit records
-      std::vector<int> sl(total), ss(total), sd(total);
-      CK(copy_async(sl.data(), ctx->rsl.p, total * sizeof(int), cudaMemcpyDeviceToHost, s));
-      CK(copy_async(sd.data(), ctx->rside.p, total * sizeof(int), cudaMemcpyDeviceToHost, s));
-      CK(cudaStreamSynchronize(s));
-      int64_t steps = 0, ng = 0, nsn = 0;
-      for (int64_t q = 0; q < total; q++) {
-        steps += sl[q];
-        if (sd[q] == -1) ng++;
-        else if (sd[q] >= 0) nsn++;
-      }
-      info->path_steps = steps;
-      info->exits_global = ng;
-      info->exits_stencil = nsn;
-    }
+    CK(launch_replay_paths(a, P.kind, ctx->num_sms, s));
+    CK(launch_replay_reduce(a, P.kind, max_n, ctx->knot_task_off.p, ctx->Gside.p, ctx->GGside.p, s));
+    launches += 5;
   } else {
     int chunks = 1, ppc = 1;
     item_split(ctx, N, &chunks, &ppc, (mode == PDDS_MODE_MIXED && tuned_for(ctx, desc)) ? ctx->tune_ppc : 0,
@@ -1368,11 +1345,9 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
     } else {
       info->paths = (int64_t)n_mc * N;
     }
-    if (mode != PDDS_MODE_REPLAY_FP64) {
-      info->path_steps = (int64_t)st[0];
-      info->exits_global = (int64_t)st[2];
-      info->exits_stencil = (int64_t)st[3];
-    }
+    info->path_steps = (int64_t)st[0];
+    info->exits_global = (int64_t)st[2];
+    info->exits_stencil = (int64_t)st[3];
     info->cta_threads = mode == PDDS_MODE_MIXED ? cta_threads_for(ctx, desc) : 0;
   }
   const pdds_status fst = check_err_flags(ctx);

@@ -156,8 +156,8 @@ struct pdds_ctx {
   bool has_estimate = false;
   // replay scratch
   DBuf<double> rx, ry, rY, rZ, rxi, Gside, GGside, ipsi_knot;
-  DBuf<int> rside, rsl, rss, task_m, task_d, task_i;
-  DBuf<int64_t> task_out, knot_task_off, knot_ipsi_off;
+  DBuf<int> rside, rsl, rss;
+  DBuf<int64_t> knot_task_off, knot_ipsi_off;
   // solve scratch
   DBuf<double> sv64, sscal, spart, shess, su;
   DBuf<float> sV32, sw32, sval32, sZ32;

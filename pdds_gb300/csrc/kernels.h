@@ -151,14 +151,16 @@ struct ReplayArgs {
   int* esteps_l;
   int* esteps_s;
   // diagnostics (all null when off): sums [K][PDDS_DIAG_N], the sublinear
-  // leg's end states [n_mc * N] and each knot's step [n_mc]
+  // leg's end states [n_mc * N]
   double* diag;
   double* sx;
   double* sy;
   double* sY;
   double* sZ;
   double* sxi;
-  double* knot_h;
+  double* knot_h;        // [n_mc][2]: each knot's step and its square root
+  unsigned long long* path_counter;  // next path to hand out
+  unsigned long long* stats;         // as in MixedArgs
   // outputs
   double* G;             // [nnz] final values
   double* GG;            // [nnz] final GG/N values (before - G^2)
@@ -193,11 +195,11 @@ bool is_mixed_path_kernel(const void* func);
 int mixed_blocks_per_sm(int kind, size_t smem, int richardson, int threads, bool diag = false);
 cudaError_t launch_paths_fp64(const Fp64Args& a, int kind, int grid, size_t smem, cudaStream_t s);
 int fp64_blocks_per_sm(int kind, size_t smem, int richardson);
-cudaError_t launch_replay_paths(const ReplayArgs& a, int kind, cudaStream_t s);
-cudaError_t launch_replay_reduce(const ReplayArgs& a, int kind, const int* task_m, const int* task_d,
-                                 const int* task_i, int ntask, const int64_t* task_out,
-                                 const int64_t* knot_task_off, double* Gside, double* GGside,
-                                 cudaStream_t s);
+cudaError_t launch_replay_paths(const ReplayArgs& a, int kind, int num_sms, cudaStream_t s);
+// max_n: side knots of the largest side; knot_task_off: first side entry of
+// each knot in Gside and GGside (sides N, S, E, W one after the other)
+cudaError_t launch_replay_reduce(const ReplayArgs& a, int kind, int max_n, const int64_t* knot_task_off,
+                                 double* Gside, double* GGside, cudaStream_t s);
 // FP64 factorisation of every shape's Psi and the cardinal-function tables.
 // lu: scratch of the ipsi layout; piv, uinv: scratch of the sh_t layout
 cudaError_t launch_rbf_setup(const DevLayout& L, int max_n, int max_nbins, double* ipsi, float* tab,
