@@ -25,6 +25,7 @@ UNITS = {
     "capi.cu": [],
     "k_mixed.cu": [],
     "k_fp64.cu": [],
+    "k_fast64.cu": [],
     "k_replay.cu": ["-fmad=false"],
     "k_rbf.cu": [],
     "k_misc.cu": ["-fmad=false"],

@@ -331,7 +331,7 @@ pdds_status upload_layout(pdds_ctx* ctx) {
     fsm = std::max(fsm, nn);
   }
   ctx->mixed_smem = msm * sizeof(float);
-  ctx->fp64_smem = (FP64_THREADS / 32 + 1) * fsm * sizeof(double);  // per-warp sums, knot coordinates
+  ctx->fp64_nall = (int)fsm;
   // the layout's arrays in one device block: one allocation and one copy
   // (a small pageable copy or an allocation costs about as much as the
   // whole 3 MB block of the 12x12/43 layout)
@@ -830,6 +830,9 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     ctx->map_owner.recycle();
     ctx->lay_block.recycle();
     ctx->sexch.recycle();
+    ctx->fast64.recycle();
+    ctx->fp64_S.recycle();
+    ctx->fp64_next.recycle();
     ctx->knot_rng.recycle();
     ctx->tab.recycle();
     ctx->lut_coef.recycle();
@@ -1258,7 +1261,6 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
     int chunks = 1, ppc = 1;
     item_split(ctx, N, &chunks, &ppc, (mode == PDDS_MODE_MIXED && tuned_for(ctx, desc)) ? ctx->tune_ppc : 0,
                cta_threads_for(ctx, desc), rn);
-    const int n_items = rn * chunks;
     CK(cudaMemsetAsync(ctx->counter.p, 0, sizeof(int), s));
     if (mode == PDDS_MODE_MIXED) {
       pdds_status st = enqueue_mixed_paths(ctx, desc, P, chunks, ppc, &launches, nullptr, r0, rn);
@@ -1268,18 +1270,22 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
         if (st != PDDS_OK) return st;
       }
     } else {
+      if (!ctx->fast64_ready) {
+        CK(ctx->fast64.resize(fast64_bytes()));
+        CK(launch_fast64_tables(ctx->fast64.p, s));
+        ++launches;
+        ctx->fast64_ready = true;
+      }
       Fp64Args a{};
       a.L = ctx->dl;
       a.P = P;
+      a.T = fast64_view(ctx->fast64.p);
       a.N = N;
       a.h = desc->h;
       a.sqrth = std::sqrt(desc->h);
       a.inv_N = 1.0 / N;
       a.seed = desc->seed;
       a.instance = desc->instance;
-      a.chunks = chunks;
-      a.paths_per_chunk = ppc;
-      a.n_items = n_items;
       a.dup_sum = ctx->L.geom == 1 ? 1 : desc->dup_sum;  // circle layouts sum shared side knots
       a.adaptive_h = desc->adaptive_h ? 1 : 0;
       a.richardson = desc->richardson ? 1 : 0;
@@ -1292,15 +1298,29 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
       a.stats = ctx->stats.p;
       a.err_flags = ctx->errf.p;
       a.diag = diag ? ctx->diag.p : nullptr;
-      const size_t smem = ctx->fp64_smem;
-      cudaFuncAttributes fa;
-      (void)fa;
-      int bps = fp64_blocks_per_sm(P.kind, smem, a.richardson);
-      if (bps < 1) bps = 1;
-      const int grid = std::max(1, std::min(n_items, bps * ctx->num_sms));
-      if (n_items > 0) {
-        CK(launch_paths_fp64(a, P.kind, grid, smem, s));
-        launches++;
+      a.blocks = chunks;
+      a.block_paths = ppc;
+      const int n_blocks = rn * chunks;
+      a.sum_stride = std::max(ctx->fp64_nall, 1);
+      CK(ctx->fp64_S.resize((size_t)std::max(n_blocks, 1) * FP64_SLOTS * a.sum_stride));
+      CK(ctx->fp64_next.resize(std::max(n_blocks, 1)));
+      CK(cudaMemsetAsync(ctx->fp64_next.p, 0, std::max(n_blocks, 1) * sizeof(int), s));
+      a.S = ctx->fp64_S.p;
+      a.next_path = ctx->fp64_next.p;
+      // a CTA takes a whole block (its lanes share the block's paths and the
+      // stencil's set-up) unless that leaves SMs without work: 19 blocks of
+      // one knot's 5,000 paths take 0.67 ms as 19 CTAs, 0.49 ms as 152
+      int slots = FP64_SLOTS;
+      while (slots > 1 && n_blocks * (FP64_SLOTS / slots) < 2 * ctx->num_sms) slots /= 2;
+      const int threads = 32 * slots;
+      const size_t smem = (size_t)(slots + 1) * a.sum_stride * sizeof(double);
+      const int bps = std::max(1, fp64_blocks_per_sm(P.kind, smem, a.richardson, threads));
+      a.n_items = n_blocks * (FP64_SLOTS / slots);
+      const int grid = std::max(1, std::min(a.n_items, bps * ctx->num_sms));
+      if (a.n_items > 0) {
+        CK(launch_paths_fp64(a, P.kind, grid, threads, smem, s));
+        CK(launch_rows_fp64(a, n_blocks, s));
+        launches += 2;
       }
     }
     if (mode == PDDS_MODE_MIXED && desc->adaptive_n)

@@ -146,7 +146,8 @@ struct pdds_ctx {
   DevLayout dl{};
   int n_mc = 0, n_bnd = 0;
   std::vector<int> mc_host;  // knots with paths, in hand-out order (the device mc_knots)
-  size_t mixed_smem = 0, fp64_smem = 0;
+  size_t mixed_smem = 0;
+  int fp64_nall = 0;              // side knots of the largest stencil
   int max_nbins = 0;
   // results and scratch
   DBuf<double> G, GG, B, BB, Bsum, BBsum;
@@ -223,6 +224,10 @@ struct pdds_ctx {
   DBuf<double> diag;              // [K][PDDS_DIAG_N] diagnostic sums of the last estimate
   bool has_diag = false;
   DBuf<double> rsx, rsy, rsY, rsZ, rsxi, rknot_h;  // replay diagnostics: sublinear ends, knot steps
+  DBuf<unsigned char> fast64;     // tables of the FP64 path kernel, filled by the first FP64 estimate
+  bool fast64_ready = false;
+  DBuf<double> fp64_S;            // RBF sums of the FP64 path kernel
+  DBuf<int> fp64_next;            // and its blocks' path counters
   DBuf<int> mc_lpt;               // MIXED hand-out order, heaviest knots first (from knot_steps)
   bool lpt_ready = false;
   bool has_knot_steps = false;

@@ -1,18 +1,35 @@
 // FP64 mode: the plain double-precision GPU form of the estimator.
 //
-// Same persistent work-item structure as the MIXED kernel, but every path
+// The paths of a knot are split into blocks of block_paths; a block is eight
+// slots of 32 lanes, slot w starting with the block's paths [32 w, 32 w + 32)
+// and every lane taking the block's next path when its own ends.  Every path
 // quantity is FP64 and each stencil exit adds its exact RBF vector
-// Y * r_j(X), r_j = exp(-|p_j - X|^2 / c^2), into per-side FP64 sums S_j in
-// shared memory.  At the end of the item G_i = -(1/N) sum_j ipsi(j,i) S_j.
+// Y * r_j(X), r_j = exp(-|p_j - X|^2 / c^2), into the FP64 sums S_j of its
+// slot.  Afterwards (k_rows_fp64) G_i = -(1/N) sum_j ipsi(j,i) S_j per block.
 // Exits are queued per warp (side, coordinate, weight) and the warp adds
 // their RBF vectors one exit at a time with the side knots spread over the
-// lanes, into its own copy of the sums (no atomics; the copies are added at
-// the end of the item), so the n_s exponentials of an exit run at full width.
+// lanes (no atomics), so the n_s exponentials of an exit run at full width.
 // By linearity this equals the reference's per-exit
 // H_i = sum_j ipsi(j,i) RBF(p_j, X) accumulation (Meshes/stencil.cpp:244-307)
 // with n_s instead of n_s^2 exponentials per exit.  It is the all-FP64 GPU
 // oracle that MIXED results are compared with.
+//
+// What bounds it: the FP64 pipe (one warp instruction per 64 cycles and
+// scheduler).  A CTA takes all eight slots of a block where there are enough
+// blocks to fill the GPU, and fewer of them where there are not (one knot of
+// 5,000 paths: 19 blocks, 152 CTAs of one warp); coefficients that reach only
+// the sums of B come from tables (fast64.cuh); the exit test of
+// constant-sigma kinds compares |x - c| with an edge formed once, as
+// integers; the normals of odd and even steps come from one place, so lanes
+// of both kinds do not run it twice.  What reaches the sums S keeps its
+// rounding and its order (positions, exponentials, the slots' sums): Psi^-1
+// has entries of 1e9 and more, so G carries the rounding of S and of the
+// product with it, and another grouping of the paths moves G by more than
+// the Monte Carlo noise of two runs.
+// 4x4/n11, N = 1e4, h = 1e-3: 49.7 -> 24.8 ms; one knot of 5,000 paths
+// 1.02 -> 0.49 ms.
 #include "dev_common.cuh"
+#include "fast64.cuh"
 #include "kernels.h"
 
 namespace pdds {
@@ -27,8 +44,6 @@ struct ItemSide64 {
   double origin;
   double inv_c2;
   int64_t t_off;     // shape's local knot coordinates
-  int64_t ipsi_off;
-  int64_t map_off;
   double R;          // arc radius (polar stencils): RBF distance = chord 2 R sin(dt / 2)
 };
 
@@ -37,7 +52,7 @@ constexpr unsigned FULL = 0xffffffffu;
 struct Lvl64 {
   double x, y, Y, Z, xi;
   double phi;  // Z + Y g(X_tau) at the exit (diagnostics)
-  Coef<double> k;
+  Coef<double> k;  // kinds whose sigma varies: the coefficients at (x, y)
   unsigned steps;
 };
 
@@ -51,38 +66,114 @@ __device__ __forceinline__ void normals_f64(uint32_t ua, uint32_t ub, double& z0
   z1 = rho * sn;
 }
 
+// Kinds with sigma = S I and no drift.
+template <int KIND>
+constexpr bool iso64 = KIND != PK_VARCOEF && !is_lut_kind(KIND);
+template <int KIND>
+constexpr double sigma64 = KIND == PK_MONEGROS ? 1.41421356237 : 1.4142135623730951;
+// Kinds with a reaction term.
+template <int KIND>
+constexpr bool react64 = KIND == PK_HELMHOLTZ || KIND == PK_VARCOEF || is_lut_kind(KIND);
+
+// coef_f64 with the table functions in the terms that reach only the sums
+// of B (f and grad u); sigma, b and c keep coef_f64's rounding.
+template <int KIND>
+__device__ __forceinline__ void coef_t64(const ProblemDev& P, const Fast64& T, double x, double y, Coef<double>& k) {
+  const double PI = 3.141592653589793;
+  if constexpr (KIND == PK_POISSON_SINCOS) {
+    double sx, cx, sy, cy;
+    f64::sincospi(T, x, sx, cx);
+    f64::sincospi(T, y, sy, cy);
+    k.f = 19.739208802178716 * (sx * cy);
+    k.g0 = fma(PI, cx * cy, y);
+    k.g1 = fma(-PI, sx * sy, x);
+    k.c = 0.0;
+  } else if constexpr (KIND == PK_HELMHOLTZ) {
+    const double a = P.p[0], b = P.p[1], c = P.p[2];
+    double sa, ca, sb, cb;
+    f64::sincos(T, a * x, sa, ca);
+    f64::sincos(T, b * y, sb, cb);
+    k.f = ((a * a + b * b) - c) * (sa * cb);
+    k.g0 = a * (ca * cb);
+    k.g1 = -(b * (sa * sb));
+    k.c = c;
+  } else if constexpr (KIND == PK_VARCOEF) {
+    const double s1 = 1.0 + 0.5 * (x * x), s2 = 1.0 + 0.5 * (y * y);
+    double sn, cs;
+    f64::sincos(T, 2.0 * y, sn, cs);
+    const double ex = f64::exp(T, x);
+    const double ux = ex * cs, uy = -2.0 * (ex * sn), uxx = ux, uyy = -4.0 * ux;
+    const double c = -(1.0 + x * x + y * y);
+    k.s00 = s1; k.s01 = 0.0; k.s10 = 0.0; k.s11 = s2;
+    k.b0 = y; k.b1 = -x; k.c = c;
+    k.f = -(0.5 * (s1 * s1 * uxx + s2 * s2 * uyy) + (y * ux - x * uy) + c * (ux + 1.0));
+    k.g0 = ux;
+    k.g1 = uy;
+  } else {
+    coef_f64<KIND>(P, x, y, k);
+  }
+  if (!P.use_cv) { k.g0 = 0.0; k.g1 = 0.0; }
+}
+// u_f64 likewise (the values of exits on the global boundary)
+template <int KIND>
+__device__ __forceinline__ double u_t64(const ProblemDev& P, const Fast64& T, double x, double y) {
+  if constexpr (KIND == PK_POISSON_SINCOS) {
+    double sx, cx, sy, cy;
+    f64::sincospi(T, x, sx, cx);
+    f64::sincospi(T, y, sy, cy);
+    return sx * cy + x * y;
+  } else if constexpr (KIND == PK_HELMHOLTZ) {
+    double sa, ca, sb, cb;
+    f64::sincos(T, P.p[0] * x, sa, ca);
+    f64::sincos(T, P.p[1] * y, sb, cb);
+    return sa * cb;
+  } else if constexpr (KIND == PK_VARCOEF) {
+    double sn, cs;
+    f64::sincos(T, 2.0 * y, sn, cs);
+    return f64::exp(T, x) * cs + 1.0;
+  } else {
+    return u_f64<KIND>(P, x, y);
+  }
+}
+
+// |d| < edge for edge >= 0, as integers (no FP64 comparison); false for NaN
+__device__ __forceinline__ bool abs_below(double d, double edge) {
+  return (unsigned long long)(__double_as_longlong(d) & 0x7fffffffffffffffLL) <
+         (unsigned long long)__double_as_longlong(edge);
+}
+
 template <int KIND, bool RICH, int GEOM>
-__global__ void __launch_bounds__(FP64_THREADS)
+__global__ void __launch_bounds__(FP64_THREADS, is_lut_kind(KIND) ? 1 : 2)
 k_paths_fp64(const Fp64Args a) {
-  // [warps][sum n] per-warp per-side RBF sums, then [sum n] local t
-  extern __shared__ double Ssum[];
+  extern __shared__ double Ssum[];  // [warps][sum n] the slots' RBF sums, then [sum n] local t
   __shared__ double s_qs[FP64_THREADS / 32][FP64_QCAP], s_qy[FP64_THREADS / 32][FP64_QCAP];
   __shared__ int s_qd[FP64_THREADS / 32][FP64_QCAP];
   __shared__ int s_qn[FP64_THREADS / 32];
   __shared__ ItemSide64 s_side[4];
   __shared__ double s_rect[4];
-  __shared__ int s_item, s_knot, s_path_end, s_nall;
+  __shared__ int s_item, s_knot, s_nall;
   __shared__ double s_h;
-  __shared__ unsigned s_next_path;
   __shared__ double s_red[FP64_THREADS / 32][2];
   __shared__ double s_diag[PDDS_DIAG_N];
   __shared__ unsigned long long s_redi[FP64_THREADS / 32][3];
   const DevLayout& L = a.L;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nthr = blockDim.x, NW = nthr >> 5;  // NW slots of a block
 
   for (;;) {
     if (tid == 0) s_item = atomicAdd(a.item_counter, 1);
     __syncthreads();
     const int item = s_item;
     if (item >= a.n_items) break;
+    // item = (block, group of NW slots); block = (knot, chunk of paths)
+    const int groups = FP64_SLOTS / NW;
+    const int block = item / groups, slot = (item - block * groups) * NW + warp;
+    const int kn = block / a.blocks, p0 = (block - kn * a.blocks) * a.block_paths;
+    const int path_end = min(a.N, p0 + a.block_paths);
     if (tid == 0) {
-      const int k = a.mc_knots[item / a.chunks];
-      const int chunk = item % a.chunks;
+      const int k = a.mc_knots[kn];
       s_knot = k;
       for (int q = 0; q < PDDS_DIAG_N; q++) s_diag[q] = 0.0;
-      const int p0 = chunk * a.paths_per_chunk;
-      s_path_end = min(a.N, p0 + a.paths_per_chunk);
-      s_next_path = (unsigned)(p0 + FP64_THREADS);
       const int st = L.knot_stencil[k];
       for (int q = 0; q < 4; q++) s_rect[q] = L.st_rect[4 * st + q];
       s_h = a.h;
@@ -93,15 +184,13 @@ k_paths_fp64(const Fp64Args a) {
                         : adaptive_step<double>(L.st_rect + 4 * st, L.kx[k], L.ky[k], a.h, kd);
       }
       int off = 0;
-      int64_t moff = L.st_map_off[st];
       for (int d = 0; d < 4; d++) {
         const int sd = L.st_side[4 * st + d];
         ItemSide64 is;
         is.glob = L.st_glob[4 * st + d];
-        is.map_off = moff;
         if (sd < 0) {
           is.n = 0; is.orient = 0; is.s_off = off; is.origin = 0.0; is.inv_c2 = 0.0;
-          is.t_off = 0; is.ipsi_off = 0; is.R = 0.0;
+          is.t_off = 0; is.R = 0.0;
         } else {
           const int sh = L.sd_shape[sd];
           is.n = L.sd_n[sd];
@@ -116,24 +205,21 @@ k_paths_fp64(const Fp64Args a) {
           const double c = L.sh_c[sh];
           is.inv_c2 = 1.0 / (c * c);
           is.t_off = L.sh_t_off[sh];
-          is.ipsi_off = L.sh_ipsi_off[sh];
           off += is.n;
-          moff += is.n;
         }
         s_side[d] = is;
       }
       s_nall = off;
     }
     __syncthreads();
-    const int knot = s_knot, path_end = s_path_end, nall = s_nall;
+    const int knot = s_knot, nall = s_nall;
     const double h = s_h, sqrth = ::sqrt(s_h);
-    constexpr int NW = FP64_THREADS / 32;
     double* tloc = Ssum + NW * nall;
     double* Sw = Ssum + warp * nall;  // this warp's sums
-    for (int i = tid; i < NW * nall; i += FP64_THREADS) Ssum[i] = 0.0;
+    for (int i = tid; i < NW * nall; i += nthr) Ssum[i] = 0.0;
     if (lane == 0) s_qn[warp] = 0;
     for (int d = 0; d < 4; d++)
-      for (int i = tid; i < s_side[d].n; i += FP64_THREADS)
+      for (int i = tid; i < s_side[d].n; i += nthr)
         tloc[s_side[d].s_off + i] = L.sh_t[s_side[d].t_off + i];
     __syncthreads();
 
@@ -151,10 +237,17 @@ k_paths_fp64(const Fp64Args a) {
     else if (rmask & 2) { rn1 = -1.0; rc = -rect[1]; }
     else if (rmask & 4) { rn0 = 1.0; rc = rect[2]; }
     else if (rmask & 8) { rn0 = -1.0; rc = -rect[0]; }
+    const Fast64& T = a.T;
+    constexpr double S = iso64<KIND> ? sigma64<KIND> : 1.0;
+    const double hf = 0.5 * h, sqf = ::sqrt(hf);
+    const double cx = 0.5 * (rect[0] + rect[2]), cy = 0.5 * (rect[1] + rect[3]);
+    // constant sigma: a path is inside while |x - cx| < ex and |y - cy| < ey
+    const double thr_c = -0.5826 * S * sqrth, thr_f = -0.5826 * S * sqf;
+    const double exc = ::fmax((rect[2] - cx) + thr_c, 0.0), eyc = ::fmax((rect[3] - cy) + thr_c, 0.0);
+    const double exf = ::fmax((rect[2] - cx) + thr_f, 0.0), eyf = ::fmax((rect[3] - cy) + thr_f, 0.0);
     Coef<double> k0;
-    coef_f64<KIND>(a.P, x0, y0, k0);
-    const int chunk = item % a.chunks;
-    unsigned path = (unsigned)(chunk * a.paths_per_chunk + tid);
+    if constexpr (!iso64<KIND>) coef_t64<KIND>(a.P, T, x0, y0, k0);
+    unsigned path = (unsigned)(p0 + 32 * slot + lane);
     bool active = (int)path < path_end;
     double b = 0.0, bb = 0.0;
     unsigned long long nsteps = 0, nglob = 0, nsten = 0;
@@ -169,10 +262,10 @@ k_paths_fp64(const Fp64Args a) {
       }
       if (glob) {
         ++nglob;
-        s.phi = s.Z + s.Y * u_f64<KIND>(a.P, Ex, Ey);
+        s.phi = s.Z + s.Y * u_t64<KIND>(a.P, T, Ex, Ey);
         return s.phi + s.xi;
       }
-      if (a.diag) s.phi = s.Z + s.Y * u_f64<KIND>(a.P, Ex, Ey);
+      if (a.diag) s.phi = s.Z + s.Y * u_t64<KIND>(a.P, T, Ex, Ey);
       ++nsten;
       if (d < 0) {
         atomicOr(a.err_flags, ERR_FLAG_EXIT_SIDE);
@@ -199,7 +292,7 @@ k_paths_fp64(const Fp64Args a) {
         const double sc = s_qs[warp][e], yw = s_qy[warp][e];
         for (int j = lane; j < is.n; j += 32) {
           const double dt0 = tloc[is.s_off + j] - sc;
-          const double dt = is.R > 0.0 ? 2.0 * is.R * ::sin(0.5 * dt0) : dt0;
+          const double dt = GEOM == 1 && is.R > 0.0 ? 2.0 * is.R * ::sin(0.5 * dt0) : dt0;
           Sw[is.s_off + j] += yw * ::exp(-(dt * dt) * is.inv_c2);
         }
       }
@@ -207,39 +300,56 @@ k_paths_fp64(const Fp64Args a) {
       if (lane == 0) s_qn[warp] = 0;
       __syncwarp();
     };
-    // ex: Exp(1) sample of the reflected step (PK_ROBIN), see k_mixed.cu
-    auto step_level = [&](Lvl64& s, double i0, double i1, double hh, double sq, double wgt, double& val,
-                          double ex) -> bool {
-      const double v0 = -(s.k.s00 * s.k.g0 + s.k.s10 * s.k.g1);
-      const double v1 = -(s.k.s01 * s.k.g0 + s.k.s11 * s.k.g1);
-      s.xi += s.Y * (v0 * i0 + v1 * i1);
-      s.Z += s.k.f * s.Y * hh;
-      s.Y += s.k.c * s.Y * hh;
-      if constexpr (KIND == PK_ROBIN) {
-        const double d0 = s.k.s00 * i0, d1 = s.k.s11 * i1;
-        double dL = 0.0;
-        if (rmask) {
-          const double dR = rn0 * s.x + rn1 * s.y - rc;
-          const double U = rn0 * d0 + rn1 * d1;
-          const double M = 0.5 * (U + ::sqrt(U * U + 4.0 * hh * ex));  // |sigma^T n|^2 = 2
-          dL = ::fmax(0.0, M + dR);
-          if (dL > 0.0) {  // exact in dL, as in k_mixed.cu
-            double vphi, psi;
-            robin_data<double>(s.x - dR * rn0, s.y - dR * rn1, rn0, rn1, vphi, psi);
-            const double t = vphi * dL;
-            const double em1 = ::expm1(t);
-            s.Z += psi * s.Y * (t != 0.0 ? em1 / vphi : dL);
-            s.Y += s.Y * em1;
-          }
+    // One step of a level with the increments i0, i1 = sqrt(h) z and its
+    // exit; ex, ey: the level's exit edges.
+    // exs: Exp(1) sample of the reflected step (PK_ROBIN), see k_mixed.cu
+    auto step_level = [&](Lvl64& s, double i0, double i1, double hh, double sq, double ex, double ey, double wgt,
+                          double& val, double exs) -> bool {
+      if constexpr (iso64<KIND>) {
+        Coef<double> k;
+        coef_t64<KIND>(a.P, T, s.x, s.y, k);
+        const double d0 = __dmul_rn(S, i0), d1 = __dmul_rn(S, i1);
+        const double gd = fma(k.g0, d0, k.g1 * d1);
+        if constexpr (react64<KIND> || KIND == PK_ROBIN) {
+          s.xi = fma(-s.Y, gd, s.xi);
+          s.Z = fma(k.f * s.Y, hh, s.Z);
+          if constexpr (react64<KIND>) s.Y = fma(k.c * s.Y, hh, s.Y);
+        } else {  // Y stays 1
+          s.xi -= gd;
+          s.Z = fma(k.f, hh, s.Z);
         }
-        s.x += d0 - dL * rn0;
-        s.y += d1 - dL * rn1;
+        if constexpr (KIND == PK_ROBIN) {
+          double dL = 0.0;
+          if (rmask) {
+            const double dR = rn0 * s.x + rn1 * s.y - rc;
+            const double U = rn0 * d0 + rn1 * d1;
+            const double M = 0.5 * (U + ::sqrt(U * U + 4.0 * hh * exs));  // |sigma^T n|^2 = 2
+            dL = ::fmax(0.0, M + dR);
+            if (dL > 0.0) {  // exact in dL, as in k_mixed.cu
+              double vphi, psi;
+              robin_data<double>(s.x - dR * rn0, s.y - dR * rn1, rn0, rn1, vphi, psi);
+              const double t = vphi * dL;
+              const double em1 = ::expm1(t);
+              s.Z += psi * s.Y * (t != 0.0 ? em1 / vphi : dL);
+              s.Y += s.Y * em1;
+            }
+          }
+          s.x += d0 - dL * rn0;
+          s.y += d1 - dL * rn1;
+        } else {
+          s.x = __dadd_rn(s.x, d0);
+          s.y = __dadd_rn(s.y, d1);
+        }
       } else {
-        s.x += s.k.b0 * hh + (s.k.s00 * i0 + s.k.s01 * i1);
-        s.y += s.k.b1 * hh + (s.k.s10 * i0 + s.k.s11 * i1);
+        const double d0 = __dmul_rn(s.k.s00, i0), d1 = __dmul_rn(s.k.s11, i1);
+        s.xi = fma(-s.Y, fma(s.k.g0, d0, s.k.g1 * d1), s.xi);
+        s.Z = fma(s.k.f * s.Y, hh, s.Z);
+        s.Y = fma(s.k.c * s.Y, hh, s.Y);
+        s.x += fma(s.k.b0, hh, d0);
+        s.y += fma(s.k.b1, hh, d1);
+        coef_t64<KIND>(a.P, T, s.x, s.y, s.k);
       }
       ++s.steps;
-      coef_f64<KIND>(a.P, s.x, s.y, s.k);
       if constexpr (GEOM == 1) {
         // polar stencil, isotropic sigma: outside distances beyond the inner
         // arc (none at the centre), the outer arc and the two rays
@@ -254,7 +364,7 @@ k_paths_fp64(const Fp64Args a) {
         if (d_out > mx) { mx = d_out; d = 0; }
         if (d_a > mx) { mx = d_a; d = 3; }
         if (d_b > mx) { mx = d_b; d = 2; }
-        if (mx < -0.5826 * ::fabs(s.k.s00) * sq) {
+        if (mx < -0.5826 * S * sq) {
           if (s.steps < (unsigned)a.max_steps) return false;
           atomicOr(a.err_flags, ERR_FLAG_STEP_LIMIT);
           val = 0.0;
@@ -295,17 +405,26 @@ k_paths_fp64(const Fp64Args a) {
         val = exit_level(s, wgt, Ex, Ey, d, s_side[d].glob != 0, s_side[d].orient == 0 ? Ex : Ey);
         return true;
       } else {
-        double Ex, Ey, Nx, Ny;
-        int onmask;
-        const double dist = rect2d<double>(rect, s.x, s.y, Ex, Ey, Nx, Ny, onmask);
-        const double w0 = Nx * s.k.s00 + Ny * s.k.s10, w1 = Nx * s.k.s01 + Ny * s.k.s11;
-        const double thr = -0.5826 * ::sqrt(w0 * w0 + w1 * w1) * sq;
-        if (dist < thr) {
+        // inside: the larger of |x - cx| - hx and |y - cy| - hy is below the
+        // threshold -0.5826 |N^T sigma| sqrt(h), N the normal of that side
+        // (beyond a corner the distance is positive and the threshold is not)
+        bool inside;
+        if constexpr (iso64<KIND>) {
+          inside = abs_below(s.x - cx, ex) && abs_below(s.y - cy, ey);
+        } else {
+          const double dx = ::fabs(s.x - cx) - (rect[2] - cx), dy = ::fabs(s.y - cy) - (rect[3] - cy);
+          const bool xs = dx > dy;
+          inside = (xs ? dx : dy) < -0.5826 * ::fabs(xs ? s.k.s00 : s.k.s11) * sq;
+        }
+        if (inside) {
           if (s.steps < (unsigned)a.max_steps) return false;
           atomicOr(a.err_flags, ERR_FLAG_STEP_LIMIT);
           val = 0.0;
           return true;
         }
+        double Ex, Ey, Nx, Ny;
+        int onmask;
+        rect2d<double>(rect, s.x, s.y, Ex, Ey, Nx, Ny, onmask);
         const int d = exit_side(onmask);
         const bool glob = ((onmask & 1) && s_side[0].glob) || ((onmask & 2) && s_side[1].glob) ||
                           ((onmask & 4) && s_side[2].glob) || ((onmask & 8) && s_side[3].glob);
@@ -315,7 +434,8 @@ k_paths_fp64(const Fp64Args a) {
     };
     Lvl64 fine, coarse;
     auto reset = [&]() {
-      fine.x = x0; fine.y = y0; fine.Y = 1.0; fine.Z = 0.0; fine.xi = 0.0; fine.phi = 0.0; fine.k = k0;
+      fine.x = x0; fine.y = y0; fine.Y = 1.0; fine.Z = 0.0; fine.xi = 0.0; fine.phi = 0.0;
+      if constexpr (!iso64<KIND>) fine.k = k0;
       fine.steps = 0;
       coarse = fine;
     };
@@ -341,12 +461,11 @@ k_paths_fp64(const Fp64Args a) {
             x1e = -::log(u01_fp64(bx.v[1]));
             x2e = -::log(u01_fp64(bx.v[2]));
           }
-          const double hf = 0.5 * h, sqf = ::sqrt(hf);
-          if (fine_alive) fine_alive = !step_level(fine, sqf * za0, sqf * za1, hf, sqf, 2.0, val_f, x0e);
-          if (fine_alive) fine_alive = !step_level(fine, sqf * zb0, sqf * zb1, hf, sqf, 2.0, val_f, x1e);
+          if (fine_alive) fine_alive = !step_level(fine, sqf * za0, sqf * za1, hf, sqf, exf, eyf, 2.0, val_f, x0e);
+          if (fine_alive) fine_alive = !step_level(fine, sqf * zb0, sqf * zb1, hf, sqf, exf, eyf, 2.0, val_f, x1e);
           if (coarse_alive)
-            coarse_alive =
-                !step_level(coarse, sqf * (za0 + zb0), sqf * (za1 + zb1), h, sqrth, -1.0, val_c, x2e);
+            coarse_alive = !step_level(coarse, sqf * (za0 + zb0), sqf * (za1 + zb1), h, sqrth, exc, eyc, -1.0, val_c,
+                                       x2e);
           if (!fine_alive && !coarse_alive) {
             const double v = 2.0 * val_f - val_c;
             b += v;
@@ -360,15 +479,14 @@ k_paths_fp64(const Fp64Args a) {
         } else {
           if ((m & 1u) == 0) blk = path_block(a.seed, a.instance, knot_word(a.L, knot), path, m >> 1);
           double z0, z1;
-          if (m & 1u) normals_f64(blk.v[2], blk.v[3], z0, z1);
-          else normals_f64(blk.v[0], blk.v[1], z0, z1);
+          normals_f64(m & 1u ? blk.v[2] : blk.v[0], m & 1u ? blk.v[3] : blk.v[1], z0, z1);
           double xe = 0.0;
           if (KIND == PK_ROBIN && rmask) {
             const u32x4 bx = path_block(a.seed, a.instance, knot_word(a.L, knot) | 0x80000000u, path, m >> 1);
             xe = -::log(u01_fp64(bx.v[m & 1u]));
           }
           ++m;
-          if (step_level(fine, sqrth * z0, sqrth * z1, h, sqrth, 1.0, val_f, xe)) {
+          if (step_level(fine, sqrth * z0, sqrth * z1, h, sqrth, exc, eyc, 1.0, val_f, xe)) {
             b += val_f;
             bb += val_f * val_f;
             nsteps += fine.steps;
@@ -377,7 +495,7 @@ k_paths_fp64(const Fp64Args a) {
           }
         }
         if (fin) {
-          path = atomicAdd(&s_next_path, 1u);
+          path = (unsigned)(p0 + 32 * FP64_SLOTS) + (unsigned)atomicAdd(a.next_path + block, 1);
           if ((int)path >= path_end) {
             active = false;
           } else {
@@ -392,11 +510,10 @@ k_paths_fp64(const Fp64Args a) {
     }
     flush(1);
     __syncthreads();
-    // S_j: the warps' sums added in a fixed order, into warp 0's copy
-    for (int i = tid; i < nall; i += FP64_THREADS) {
-      double t = Ssum[i];
-      for (int w = 1; w < NW; w++) t += Ssum[w * nall + i];
-      Ssum[i] = t;
+    // the slot's sums
+    {
+      double* out = a.S + ((int64_t)block * FP64_SLOTS + slot) * a.sum_stride;
+      for (int i = lane; i < nall; i += 32) out[i] = Sw[i];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -417,7 +534,7 @@ k_paths_fp64(const Fp64Args a) {
     if (tid == 0) {
       double tb = 0.0, tbb = 0.0;
       unsigned long long ts = 0, tg = 0, tt = 0;
-      for (int w = 0; w < FP64_THREADS / 32; w++) {
+      for (int w = 0; w < NW; w++) {
         tb += s_red[w][0]; tbb += s_red[w][1];
         ts += s_redi[w][0]; tg += s_redi[w][1]; tt += s_redi[w][2];
       }
@@ -428,32 +545,69 @@ k_paths_fp64(const Fp64Args a) {
       atomicAdd(a.stats + 3, tt);
     }
     if (a.diag) diag_flush(s_diag, a.diag + (int64_t)knot * PDDS_DIAG_N, tid);
-    // G_i = -(1/N) sum_j ipsi(j,i) S_j
-    const int64_t row0 = L.row_ptr[knot];
-    for (int pr = tid; pr < nall; pr += FP64_THREADS) {
-      int d = 0, i = pr;
-      while (i >= s_side[d].n) { i -= s_side[d].n; ++d; }
-      const ItemSide64& is = s_side[d];
-      const int64_t m = is.map_off + i;
-      if (!a.dup_sum && !L.map_owner[m]) continue;
-      const double* ip = L.ipsi + is.ipsi_off + i;
-      double acc = 0.0;
-      for (int j = 0; j < is.n; j++) acc += ip[(int64_t)j * is.n] * Ssum[is.s_off + j];
-      if (idx_ok(L.map_pos[m], L.row_ptr[knot + 1] - row0, a.err_flags))
-        atomicAdd(a.G + row0 + L.map_pos[m], -acc * a.inv_N);
-    }
     __syncthreads();
+  }
+}
+
+// G_i = -(1/N) sum_j ipsi(j,i) S_j of one block of paths, S_j the slots'
+// sums added in order.
+constexpr int ROWS64_THREADS = 128;
+__global__ void __launch_bounds__(ROWS64_THREADS) k_rows_fp64(const Fp64Args a) {
+  extern __shared__ double S[];
+  __shared__ int s_n[4], s_soff[4];
+  __shared__ int64_t s_ip[4], s_map[4];
+  const DevLayout& L = a.L;
+  const int block = blockIdx.x, tid = threadIdx.x;
+  const int knot = a.mc_knots[block / a.blocks];
+  const int st = L.knot_stencil[knot];
+  if (tid == 0) {
+    int off = 0;
+    int64_t moff = L.st_map_off[st];
+    for (int d = 0; d < 4; d++) {
+      const int sd = L.st_side[4 * st + d];
+      s_n[d] = sd < 0 ? 0 : L.sd_n[sd];
+      s_soff[d] = off;
+      s_map[d] = moff;
+      s_ip[d] = sd < 0 ? 0 : L.sh_ipsi_off[L.sd_shape[sd]];
+      off += s_n[d];
+      moff += s_n[d];
+    }
+  }
+  __syncthreads();
+  const int nall = s_soff[3] + s_n[3];
+  const double* src = a.S + (int64_t)block * FP64_SLOTS * a.sum_stride;
+  for (int i = tid; i < nall; i += ROWS64_THREADS) {
+    double t = src[i];
+#pragma unroll
+    for (int w = 1; w < FP64_SLOTS; w++) t += src[w * a.sum_stride + i];
+    S[i] = t;
+  }
+  __syncthreads();
+  const int64_t row0 = L.row_ptr[knot];
+  for (int pr = tid; pr < nall; pr += ROWS64_THREADS) {
+    int d = 0, i = pr;
+    while (i >= s_n[d]) { i -= s_n[d]; ++d; }
+    const int n = s_n[d];
+    const int64_t mp = s_map[d] + i;
+    if (!a.dup_sum && !L.map_owner[mp]) continue;
+    const double* ip = L.ipsi + s_ip[d] + i;
+    const double* Sd = S + s_soff[d];
+    double acc = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < n; j++) acc = fma(__ldg(ip + (int64_t)j * n), Sd[j], acc);
+    if (idx_ok(L.map_pos[mp], L.row_ptr[knot + 1] - row0, a.err_flags))
+      atomicAdd(a.G + row0 + L.map_pos[mp], -acc * a.inv_N);
   }
 }
 
 }  // namespace
 
 template <bool RICH>
-static cudaError_t launch_fp64_t(const Fp64Args& a, int kind, int grid, size_t smem, cudaStream_t s) {
+static cudaError_t launch_fp64_t(const Fp64Args& a, int kind, int grid, int threads, size_t smem, cudaStream_t s) {
 #define PDDS_FP64_CASE(KK, GG)                                                                           \
   case KK:                                                                                               \
     cudaFuncSetAttribute(k_paths_fp64<KK, RICH, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    k_paths_fp64<KK, RICH, GG><<<grid, FP64_THREADS, smem, s>>>(a);                                      \
+    k_paths_fp64<KK, RICH, GG><<<grid, threads, smem, s>>>(a);                                      \
     break;
   if (a.L.geom == 1) {
     switch (kind) {
@@ -477,26 +631,32 @@ static cudaError_t launch_fp64_t(const Fp64Args& a, int kind, int grid, size_t s
   return cudaGetLastError();
 }
 
-cudaError_t launch_paths_fp64(const Fp64Args& a, int kind, int grid, size_t smem, cudaStream_t s) {
-  return a.richardson ? launch_fp64_t<true>(a, kind, grid, smem, s) : launch_fp64_t<false>(a, kind, grid, smem, s);
+cudaError_t launch_paths_fp64(const Fp64Args& a, int kind, int grid, int threads, size_t smem, cudaStream_t s) {
+  return a.richardson ? launch_fp64_t<true>(a, kind, grid, threads, smem, s)
+                      : launch_fp64_t<false>(a, kind, grid, threads, smem, s);
+}
+
+cudaError_t launch_rows_fp64(const Fp64Args& a, int n_blocks, cudaStream_t s) {
+  k_rows_fp64<<<n_blocks, ROWS64_THREADS, a.sum_stride * sizeof(double), s>>>(a);
+  return cudaGetLastError();
 }
 
 template <bool RICH>
-static int blocks64_t(int kind, size_t smem) {
+static int blocks64_t(int kind, size_t smem, int threads) {
   int nb = 0;
   switch (kind) {
-    case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<0, RICH, 0>, FP64_THREADS, smem); break;
-    case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<1, RICH, 0>, FP64_THREADS, smem); break;
-    case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<2, RICH, 0>, FP64_THREADS, smem); break;
-    case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<4, RICH, 0>, FP64_THREADS, smem); break;
-    case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<5, RICH, 0>, FP64_THREADS, smem); break;
-    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<3, RICH, 0>, FP64_THREADS, smem); break;
+    case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<0, RICH, 0>, threads, smem); break;
+    case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<1, RICH, 0>, threads, smem); break;
+    case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<2, RICH, 0>, threads, smem); break;
+    case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<4, RICH, 0>, threads, smem); break;
+    case 5: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<5, RICH, 0>, threads, smem); break;
+    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_fp64<3, RICH, 0>, threads, smem); break;
   }
   return nb;
 }
 
-int fp64_blocks_per_sm(int kind, size_t smem, int richardson) {
-  return richardson ? blocks64_t<true>(kind, smem) : blocks64_t<false>(kind, smem);
+int fp64_blocks_per_sm(int kind, size_t smem, int richardson, int threads) {
+  return richardson ? blocks64_t<true>(kind, smem, threads) : blocks64_t<false>(kind, smem, threads);
 }
 
 }  // namespace pdds

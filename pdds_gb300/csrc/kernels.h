@@ -5,6 +5,7 @@
 
 #include "../../include/pdds.h"
 #include "dev_common.cuh"
+#include "fast64.cuh"
 
 namespace pdds {
 
@@ -13,7 +14,8 @@ constexpr int MIXED_MAX_THREADS = 256;
 // layouts, where they were faster (12x12/n43: 27.7 against 28.2 ms), 256
 // (4 per SM) below 8192 Monte Carlo knots, where 128 measured 6-17 % slower.
 inline int mixed_threads(int n_mc) { return n_mc >= 8192 ? 128 : 256; }
-constexpr int FP64_THREADS = 256;
+constexpr int FP64_SLOTS = 8;      // warps that share a block of paths in the FP64 kernel
+constexpr int FP64_THREADS = 32 * FP64_SLOTS;  // at most (a CTA may take fewer slots)
 constexpr int FP64_QCAP = 96;  // exits queued per warp in the FP64 kernel
 constexpr unsigned ERR_FLAG_STEP_LIMIT = 1u;
 constexpr unsigned ERR_FLAG_EXIT_SIDE = 2u;
@@ -107,17 +109,22 @@ struct MixedArgs {
 struct Fp64Args {
   DevLayout L;
   ProblemDev P;
+  Fast64 T;
   int N;
   double h, sqrth, inv_N;
   uint64_t seed;
   uint32_t instance;
-  int chunks, paths_per_chunk, n_items;
+  int blocks, block_paths;  // blocks of paths per knot, paths per block
+  int n_items;              // knots x blocks x (FP64_SLOTS / slots per CTA)
   int dup_sum;
   int adaptive_h;
   int richardson;
   long long max_steps;
   const int* mc_knots;
   int* item_counter;
+  int* next_path;           // per block, zeroed: paths handed out beyond the slots' first ones
+  double* S;                // [knots x blocks][FP64_SLOTS][sum_stride]: the slots' RBF sums
+  int sum_stride;
   double* G;
   double* Bsum;
   double* BBsum;
@@ -193,8 +200,9 @@ void portable_math_check_host(int fn, const double* x, int n, double* out);
 // nodes are re-keyed with a new seed through their parameters).
 bool is_mixed_path_kernel(const void* func);
 int mixed_blocks_per_sm(int kind, size_t smem, int richardson, int threads, bool diag = false);
-cudaError_t launch_paths_fp64(const Fp64Args& a, int kind, int grid, size_t smem, cudaStream_t s);
-int fp64_blocks_per_sm(int kind, size_t smem, int richardson);
+cudaError_t launch_paths_fp64(const Fp64Args& a, int kind, int grid, int threads, size_t smem, cudaStream_t s);
+int fp64_blocks_per_sm(int kind, size_t smem, int richardson, int threads);
+cudaError_t launch_rows_fp64(const Fp64Args& a, int n_blocks, cudaStream_t s);
 cudaError_t launch_replay_paths(const ReplayArgs& a, int kind, int num_sms, cudaStream_t s);
 // max_n: side knots of the largest side; knot_task_off: first side entry of
 // each knot in Gside and GGside (sides N, S, E, W one after the other)
