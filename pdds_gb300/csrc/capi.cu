@@ -534,6 +534,35 @@ struct ItemList {
   const double* knot_invN;
 };
 
+// Table nodes that a path-kernel CTA may stage in shared memory: the largest
+// stencil window that leaves the kernel's 512 threads per SM room, or none
+// where that covers less than half of the knots (a knot whose window is
+// larger reads its nodes through L1).  The line lies at the room because a
+// CTA less per SM costs more than L1's gathers do: tables of 256^2 nodes on
+// 8 x 8 subdomains (room for all windows) 18.4 ms through L1, 17.7 staged;
+// tables of 500^2 (four times the nodes) stay at 24.3 ms.  Returns the bytes.
+size_t lut_stage(const pdds_ctx* ctx, const ProblemDev& P, size_t base_smem, int threads, int* nodes) {
+  constexpr size_t PER_SM = 228 * 1024, FIXED = 3 * 1024;  // static and reserved shared memory of a CTA
+  *nodes = 0;
+  const size_t share = PER_SM / (512 / threads);
+  if (ctx->L.geom != 0 || share < base_smem + FIXED + 64) return 0;
+  const int64_t cap = (int64_t)((share - base_smem - FIXED - 64) / (2 * sizeof(float4)));
+  const HostLayout& L = ctx->L;
+  std::vector<int64_t> win(L.stencils.size());
+  for (size_t i = 0; i < win.size(); i++) {
+    const double* r = L.stencils[i].rect;
+    int nx = 0, ny = 0;
+    lut_window<float>((float)r[0], (float)r[2], (float)P.lut.x0, (float)P.lut.inv_dx, P.lut.nx, nx);
+    lut_window<float>((float)r[1], (float)r[3], (float)P.lut.y0, (float)P.lut.inv_dy, P.lut.ny, ny);
+    win[i] = (int64_t)nx * ny;
+    if (win[i] <= cap) *nodes = std::max(*nodes, (int)win[i]);
+  }
+  int64_t in = 0;
+  for (int v : ctx->mc_host) in += win[L.knot_stencil[v]] <= *nodes;
+  if (2 * in < (int64_t)ctx->mc_host.size()) *nodes = 0;
+  return *nodes > 0 ? (size_t)*nodes * 2 * sizeof(float4) + 16 : 0;
+}
+
 pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, const ProblemDev& P, int chunks,
                                 int ppc, int* launches, const ItemList* items = nullptr, int mc0 = 0,
                                 int mc_n = -1) {
@@ -642,9 +671,11 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   a.step_hist = desc->step_histogram ? ctx->step_hist.p : nullptr;
   a.diag = (desc->diagnostics && ctx->diag.n >= (size_t)ctx->L.K * PDDS_DIAG_N) ? ctx->diag.p : nullptr;
   const int threads = cta_threads_for(ctx, desc);
-  const size_t smem = ctx->mixed_smem * (a.want_var ? 2 : 1) + mixed_queue_smem(threads, a.richardson);
-  if (smem > 200 * 1024) return fail(ctx, PDDS_ERR_INVALID, "exit histograms exceed shared memory; lower bins_per_gap");
+  const size_t base_smem = ctx->mixed_smem * (a.want_var ? 2 : 1) + mixed_queue_smem(threads, a.richardson);
+  a.hist_cap = (int)(ctx->mixed_smem / sizeof(float));
   const int mk = mixed_kind(P);
+  const size_t smem = base_smem + (mk == PK_LUT ? lut_stage(ctx, P, base_smem, threads, &a.lut_nodes) : 0);
+  if (smem > 200 * 1024) return fail(ctx, PDDS_ERR_INVALID, "exit histograms exceed shared memory; lower bins_per_gap");
   int bps = mixed_blocks_per_sm(mk, smem, a.richardson, threads, a.diag != nullptr);
   if (bps < 1) bps = 1;
   if (ctx->force_bps > 0) bps = std::min(bps, ctx->force_bps);

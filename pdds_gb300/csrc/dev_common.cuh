@@ -137,6 +137,19 @@ __host__ __device__ __forceinline__ void lut_coord(T x, T x0, T inv_dx, int n, i
   if (i > n - 2) i = n - 2;
   t = g - T(i);
 }
+// First node and number of nodes (n_out) along one axis that samples at
+// coordinates in [a, b] read: the sampler's own index of both ends and the
+// four nodes around each.
+template <typename T>
+__host__ __device__ __forceinline__ int lut_window(T a, T b, T x0, T inv_dx, int n, int& n_out) {
+  int i0, i1;
+  T t;
+  lut_coord<T>(a, x0, inv_dx, n, i0, t);
+  lut_coord<T>(b, x0, inv_dx, n, i1, t);
+  const int lo = i0 - 1 < 0 ? 0 : i0 - 1, hi = i1 + 2 > n - 1 ? n - 1 : i1 + 2;
+  n_out = hi - lo + 1;
+  return lo;
+}
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 // One table node, its 8 fields as two float4 (32 bytes, 32-byte aligned: the
@@ -148,29 +161,25 @@ __device__ __forceinline__ void ldg_node(const float4* p, float4& a, float4& b) 
       : "l"(p));
 }
 
-// all eight fields (nf = 8) or the first four (nf = 4: sigma11, sigma22, b1, b2)
-template <typename T, int NF>
-__device__ __forceinline__ void lut_sample(const LutDev& L, T x, T y, T* out) {
-  int ix, iy;
-  T tx, ty, wx[4], wy[4];
-  lut_coord<T>(x, (T)L.x0, (T)L.inv_dx, L.nx, ix, tx);
-  lut_coord<T>(y, (T)L.y0, (T)L.inv_dy, L.ny, iy, ty);
+// all eight fields (nf = 8) or the first four (nf = 4: sigma11, sigma22, b1,
+// b2); node(yy, xx, a, b) reads a table node
+template <typename T, int NF, typename Node>
+__device__ __forceinline__ void lut_sum_nodes(const LutDev& L, int ix, int iy, T tx, T ty, T* out, Node node) {
+  T wx[4], wy[4];
   cr_weights<T>(tx, wx);
   cr_weights<T>(ty, wy);
 #pragma unroll
   for (int f = 0; f < NF; f++) out[f] = T(0);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    const float4* row = L.coef + (int64_t)2 * clampi(iy - 1 + r, 0, L.ny - 1) * L.nx;
+    const int yy = clampi(iy - 1 + r, 0, L.ny - 1);
     T acc[NF];
 #pragma unroll
     for (int f = 0; f < NF; f++) acc[f] = T(0);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      const int xx = clampi(ix - 1 + c, 0, L.nx - 1);
       float4 a, b;
-      if (NF == 8) ldg_node(row + 2 * xx, a, b);
-      else a = __ldg(row + 2 * xx);
+      node(yy, clampi(ix - 1 + c, 0, L.nx - 1), a, b);
       acc[0] += wx[c] * (T)a.x; acc[1] += wx[c] * (T)a.y; acc[2] += wx[c] * (T)a.z; acc[3] += wx[c] * (T)a.w;
       if (NF == 8) {
         acc[NF > 4 ? 4 : 0] += wx[c] * (T)b.x; acc[NF > 5 ? 5 : 0] += wx[c] * (T)b.y;
@@ -180,6 +189,22 @@ __device__ __forceinline__ void lut_sample(const LutDev& L, T x, T y, T* out) {
 #pragma unroll
     for (int f = 0; f < NF; f++) out[f] += wy[r] * acc[f];
   }
+}
+template <typename T, int NF, typename Node>
+__device__ __forceinline__ void lut_sample_nodes(const LutDev& L, T x, T y, T* out, Node node) {
+  int ix, iy;
+  T tx, ty;
+  lut_coord<T>(x, (T)L.x0, (T)L.inv_dx, L.nx, ix, tx);
+  lut_coord<T>(y, (T)L.y0, (T)L.inv_dy, L.ny, iy, ty);
+  lut_sum_nodes<T, NF>(L, ix, iy, tx, ty, out, node);
+}
+template <typename T, int NF>
+__device__ __forceinline__ void lut_sample(const LutDev& L, T x, T y, T* out) {
+  lut_sample_nodes<T, NF>(L, x, y, out, [&](int yy, int xx, float4& a, float4& b) {
+    const float4* p = L.coef + (int64_t)2 * yy * L.nx + 2 * xx;
+    if (NF == 8) ldg_node(p, a, b);
+    else a = __ldg(p);
+  });
 }
 template <typename T>
 __device__ __forceinline__ T lut_sample_g(const LutDev& L, T x, T y) {

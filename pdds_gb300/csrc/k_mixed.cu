@@ -164,6 +164,13 @@ __device__ __forceinline__ float exit_edge(float hw, float t) {
   return __uint_as_float(lo);
 }
 
+// Sampler indices i (of nodes i - 1 .. i + 2, clamped to the table's n) that
+// read only nodes [lo, lo + len).
+__device__ __forceinline__ int2 window_range(int lo, int len, int n, bool staged) {
+  if (!staged) return make_int2(1, 0);
+  return make_int2(lo == 0 ? 0 : lo + 1, lo + len == n ? n - 2 : lo + len - 3);
+}
+
 // Table-served coefficients sampled from the nodes (PK_LUT) need more live
 // registers for the bicubic accumulation: 128 registers there; the texture
 // samplers (PK_LUT_TEX) leave the interpolation to the texture units and
@@ -185,6 +192,7 @@ k_paths_mixed(const MixedArgs a) {
   __shared__ int s_item, s_knot, s_p0, s_path_end, s_hist_len;
   __shared__ float s_h, s_sqrth;
   __shared__ float s_edge[4];  // exit edges: fine x, fine y, coarse x, coarse y
+  __shared__ int s_win[4];     // staged table window: first node x, y, nodes per row, rows (0: not staged)
   __shared__ unsigned s_next_path;
   __shared__ double s_red[MIXED_MAX_THREADS / 32][4];
   __shared__ unsigned long long s_redi[MIXED_MAX_THREADS / 32][3];
@@ -299,6 +307,42 @@ k_paths_mixed(const MixedArgs a) {
     const float scc = KindTraits<KIND>::iso ? 1.41421356f * sqrth : sqrth;
     const float scf = scc * 0.70710678f;
     const float thrc = -0.5826f * scc, thrf = -0.5826f * scf;
+    // table nodes (PK_LUT): a sample is 16 gathers of 32 bytes, and a warp's
+    // scattered lanes make the L1 the bound (16 sectors a gather).  So the
+    // window that positions inside the stencil read goes to shared memory where
+    // it fits, fields 0-3 and 4-7 apart (16-byte reads, a quarter warp per
+    // access).  8 x 8 subdomains, 21 knots a side: the paths of the semilinear
+    // loop's tables (2 x 10^4 a knot) 38.8 -> 24.9 ms; varying tables (8000 a
+    // knot) of 256^2 nodes 18.4 -> 17.7 ms, of 500^2 (no room) 24.3 as before.
+    float4* tabA = nullptr;
+    bool uni = false;
+    if constexpr (KIND == PK_LUT) {
+      tabA = reinterpret_cast<float4*>(dyn + ((nwarps * QW + (a.want_var ? 2 : 1) * a.hist_cap + 3) & ~3));
+      if (tid == 0) {
+        const LutDev& T = P.lut;
+        const int bx = lut_window<float>(s_rect[0], s_rect[2], (float)T.x0, (float)T.inv_dx, T.nx, s_win[2]);
+        const int by = lut_window<float>(s_rect[1], s_rect[3], (float)T.y0, (float)T.inv_dy, T.ny, s_win[3]);
+        s_win[0] = bx;
+        s_win[1] = by;
+        if ((int64_t)s_win[2] * s_win[3] > a.lut_nodes) s_win[3] = 0;
+      }
+      __syncthreads();
+      const int n = s_win[2] * s_win[3];
+      int same = 1;
+      float4 u0, v0;
+      ldg_node(P.lut.coef + (int64_t)2 * s_win[1] * P.lut.nx + 2 * s_win[0], u0, v0);
+      for (int i = tid; i < n; i += nthr) {
+        const int yy = i / s_win[2], xx = i - yy * s_win[2];
+        float4 u, v;
+        ldg_node(P.lut.coef + (int64_t)2 * (s_win[1] + yy) * P.lut.nx + 2 * (s_win[0] + xx), u, v);
+        tabA[i] = u;
+        tabA[a.lut_nodes + i] = v;
+        same &= u.x == u0.x && u.y == u0.y && u.z == u0.z && u.w == u0.w;
+      }
+      // sigma and b the same at every node (the outer loops' tables): every
+      // lane reads node 0 for them, one broadcast instead of a gather
+      uni = __syncthreads_and(same) != 0;
+    }
     if (EDGES && tid < 4) {
       const float lo = s_rect[tid & 1], up = s_rect[2 + (tid & 1)];
       s_edge[tid] = exit_edge(up - 0.5f * (lo + up), tid < 2 && RICH ? thrf : thrc);
@@ -363,6 +407,12 @@ k_paths_mixed(const MixedArgs a) {
     unsigned* qmeta = reinterpret_cast<unsigned*>(q2 + QP);
     const bool use_cv = P.use_cv != 0;
     const unsigned maxs = (unsigned)a.max_steps;
+    // staged window: row length, offset of node (0, 0), offset of fields 4-7,
+    // and the sampler indices whose four nodes lie in it (none: not staged)
+    const int win_n = KIND == PK_LUT ? s_win[2] : 0, win_b = KIND == PK_LUT ? a.lut_nodes : 0;
+    const int win_0 = KIND == PK_LUT ? s_win[1] * win_n + s_win[0] : 0, mask_a = uni ? 0 : -1;
+    const int2 win_ix = KIND == PK_LUT ? window_range(s_win[0], s_win[2], P.lut.nx, s_win[3] > 0) : make_int2(0, 0);
+    const int2 win_iy = KIND == PK_LUT ? window_range(s_win[1], s_win[3], P.lut.ny, s_win[3] > 0) : make_int2(0, 0);
     const float2 edge_f = make_float2(s_edge[0], s_edge[1]), edge_c = make_float2(s_edge[2], s_edge[3]);
 
     // One step of a level (Step, control-variate variant,
@@ -456,7 +506,28 @@ k_paths_mixed(const MixedArgs a) {
         const float dx = fabsf(s.x - cx) - hx, dy = fabsf(s.y - cy) - hy;
         float t = thr;
         if constexpr (is_lut_kind(KIND)) {
-          lut_sample_f32<KIND, 8>(P.lut, s.x, s.y, s.cf);
+          // outside the stencil the path exits whatever sigma is (t <= 0): no
+          // sample there (texture sampler, 31 knots per side: 222.7 -> 208.0 ms)
+          if (!(fmaxf(dx, dy) < 0.f)) return true;
+          if constexpr (KIND == PK_LUT) {
+            int ix, iy;
+            float tx, ty;
+            lut_coord<float>(s.x, (float)P.lut.x0, (float)P.lut.inv_dx, P.lut.nx, ix, tx);
+            lut_coord<float>(s.y, (float)P.lut.y0, (float)P.lut.inv_dy, P.lut.ny, iy, ty);
+            // staged, unless the window's end rounds the other way for this lane
+            if (ix >= win_ix.x && ix <= win_ix.y && iy >= win_iy.x && iy <= win_iy.y)
+              lut_sum_nodes<float, 8>(P.lut, ix, iy, tx, ty, s.cf, [&](int yy, int xx, float4& u, float4& v) {
+                const int i = yy * win_n + xx - win_0;
+                u = tabA[i & mask_a];
+                v = tabA[win_b + i];
+              });
+            else
+              lut_sum_nodes<float, 8>(P.lut, ix, iy, tx, ty, s.cf, [&](int yy, int xx, float4& u, float4& v) {
+                ldg_node(P.lut.coef + (int64_t)2 * yy * P.lut.nx + 2 * xx, u, v);
+              });
+          } else {
+            lut_sample_f32<KIND, 8>(P.lut, s.x, s.y, s.cf);
+          }
           t *= dx > dy ? fabsf(s.cf[0]) : fabsf(s.cf[1]);
         } else if constexpr (!KindTraits<KIND>::iso) {
           float nx, ny;  // |N^T sigma| for the x and y normals

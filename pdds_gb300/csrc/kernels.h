@@ -85,6 +85,8 @@ struct MixedArgs {
   double h64;            // h in FP64 (for the adaptive step)
   long long max_steps;
   const int* mc_knots;   // knots that need paths, in hand-out order
+  int hist_cap;          // words reserved for one exit histogram
+  int lut_nodes;         // table nodes that can be staged in shared memory (PK_LUT)
   int* item_counter;
   double* G;             // [nnz] accumulates -sum Y H / N
   double* GG;            // [nnz] accumulates sum (Y H)^2 / N
