@@ -24,6 +24,7 @@ CU_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler
 UNITS = {
     "capi.cu": [],
     "k_mixed.cu": [],
+    "k_contract.cu": [],
     "k_fp64.cu": [],
     "k_fast64.cu": [],
     "k_replay.cu": ["-fmad=false"],

@@ -223,13 +223,19 @@ pdds_status pdds_batch_run(pdds_ctx* ctx, const pdds_batch_run_desc* desc, pdds_
   const int64_t nnz = L.row_ptr[L.K];
   const int m = std::max(2, std::min(desc->solve.restart > 0 ? desc->solve.restart : 30, GMRES_CLUSTER_MAX_M));
   // buffers first: a captured graph holds their addresses
-  const void* before[5] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p};
+  const void* before[6] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p, ctx->hist.p};
+  size_t hw = 1;
+  for (int w = 0, W = batch_waves(ctx, desc); w < W; w++) {
+    const int i0 = (int)((int64_t)ctx->n_inst * w / W), i1 = (int)((int64_t)ctx->n_inst * (w + 1) / W);
+    hw = std::max(hw, mixed_hist_words(ctx, &ed, ctx->inst_mc0[i1] - ctx->inst_mc0[i0]));
+  }
+  CK(ctx->hist.resize(hw));
   CK(ctx->sV32.resize((size_t)(m + 1) * K));
   if (desc->solve.gmres_form == PDDS_GMRES_PIPELINED) CK(ctx->sZ32.resize((size_t)(m + 1) * K));
   CK(ctx->sval32.resize(std::max<int64_t>(nnz, 1)));
   CK(ctx->sv64.resize(std::max<int64_t>(K, 1) * 6));
   CK(ctx->su.resize(std::max<int64_t>(K, 1)));
-  const void* after[5] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p};
+  const void* after[6] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p, ctx->hist.p};
   if (std::memcmp(before, after, sizeof(before)) != 0) drop_graph(ctx);
   // the graph is reused while the descriptor, the cluster size and the solve
   // scratch (which pdds_solve_interface may also reallocate) are unchanged;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -308,13 +309,14 @@ pdds_status upload_layout(pdds_ctx* ctx) {
     sh_t_off.push_back((int64_t)sh_t.size());
     for (double v : sh.t) sh_t.push_back(v);
     ipsi_len = std::max<int64_t>(ipsi_len, sh.ipsi_off + (int64_t)sh.n * sh.n);
-    tab_len = std::max<int64_t>(tab_len, sh.tab_off + (int64_t)sh.nbins * sh.n);
+    tab_len = std::max<int64_t>(tab_len, (sh.tab_off + (int64_t)sh.nbins * sh.n + 3) & ~int64_t(3));
     max_n = std::max(max_n, sh.n);
     ctx->max_nbins = std::max(ctx->max_nbins, sh.nbins);
   }
   if (max_n > 160) return fail(ctx, PDDS_ERR_INVALID, "stencil side larger than 160 knots");
   std::vector<int> mc, bnd;
   for (int v : L.order) (L.knot_boundary[v] ? bnd : mc).push_back(v);
+  ctx->max_n = max_n;
   ctx->n_mc = (int)mc.size();
   ctx->mc_host = mc;
   ctx->n_bnd = (int)bnd.size();
@@ -372,6 +374,9 @@ pdds_status upload_layout(pdds_ctx* ctx) {
   pk.add(ctx->sh_t_off, sh_t_off);
   pk.add(ctx->sh_t, sh_t);
   pk.add(ctx->mc_knots, mc);
+  std::vector<int> mc_pos(L.K, 0);
+  for (int m = 0; m < ctx->n_mc; m++) mc_pos[mc[m]] = m;
+  pk.add(ctx->mc_pos, mc_pos);
   pk.add(ctx->bnd_knots, bnd);
   if (!kr.empty()) pk.add(ctx->knot_rng, kr);
   else ctx->knot_rng.release();
@@ -525,14 +530,29 @@ void item_split(const pdds_ctx* ctx, int N, int* chunks_out, int* ppc_out, int t
   *ppc_out = ppc;
 }
 
-// explicit work items of a continuation pass (variance-adaptive paths)
+// explicit work items (a continuation pass of variance-adaptive paths, knots
+// with a reflecting side, the autotuner's samples); host: the items' knots
 struct ItemList {
   const int* knot;
   const int* p0;
   const int* p1;
   int n;
   const double* knot_invN;
+  const int* host;
 };
+
+// Words of one exit histogram and of a work item's slot (both histograms
+// when variances are asked for).
+int hist_words(const pdds_ctx* ctx) { return (int)((ctx->mixed_smem / sizeof(float) + 3) & ~size_t(3)); }
+int64_t slot_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc) {
+  return (int64_t)hist_words(ctx) * (desc->want_var ? 2 : 1);
+}
+// Device memory for the slots of one path-kernel launch; launches with more
+// work items are split (12x12/n43: 236 MB).
+constexpr int64_t HIST_MAX_BYTES = int64_t(1) << 30;
+int64_t max_slots(const pdds_ctx* ctx, const pdds_estimate_desc* desc) {
+  return std::max<int64_t>(1, HIST_MAX_BYTES / (int64_t)sizeof(float) / std::max<int64_t>(1, slot_words(ctx, desc)));
+}
 
 // Table nodes that a path-kernel CTA may stage in shared memory: the largest
 // stencil window that leaves the kernel's 512 threads per SM room, or none
@@ -568,6 +588,17 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
                                 int mc_n = -1) {
   cudaStream_t s = ctx->stream;
   if (mc_n < 0) mc_n = ctx->n_mc;
+  // more work items than histogram slots: one launch after another
+  const int64_t slots = max_slots(ctx, desc);
+  if (items && items->n > slots) {
+    for (int i = 0; i < items->n; i += (int)slots) {
+      const ItemList part{items->knot + i, items->p0 + i, items->p1 + i, (int)std::min<int64_t>(slots, items->n - i),
+                          items->knot_invN, items->host + i};
+      const pdds_status st = enqueue_mixed_paths(ctx, desc, P, chunks, ppc, launches, &part);
+      if (st != PDDS_OK) return st;
+    }
+    return PDDS_OK;
+  }
   if (!items && P.kind == PK_ROBIN && (int)P.p[0] != 0 && !ctx->is_batch && mc0 == 0 && mc_n == ctx->n_mc) {
     // Knots whose stencil has a reflecting side take several times the
     // steps per path of the others (their paths leave only through the
@@ -601,8 +632,17 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
     CK(ctx->item_knot.upload(ik, s));
     CK(ctx->item_p0.upload(ip0, s));
     CK(ctx->item_p1.upload(ip1, s));
-    const ItemList il{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), nullptr};
+    const ItemList il{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), nullptr, ik.data()};
     return enqueue_mixed_paths(ctx, desc, P, 1, ppc, launches, &il);
+  }
+  if (!items && (int64_t)mc_n * chunks > slots && mc_n > 1) {
+    const int part = (int)std::max<int64_t>(1, std::min<int64_t>(mc_n - 1, slots / chunks));
+    for (int m = 0; m < mc_n; m += part) {
+      const pdds_status st =
+          enqueue_mixed_paths(ctx, desc, P, chunks, ppc, launches, nullptr, mc0 + m, std::min(part, mc_n - m));
+      if (st != PDDS_OK) return st;
+    }
+    return PDDS_OK;
   }
   const int N = desc->npaths;
   const int n_items = items ? items->n : mc_n * chunks;
@@ -614,13 +654,11 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   a.N = N;
   a.h = (float)desc->h;
   a.sqrth = (float)std::sqrt(desc->h);
-  a.inv_N = 1.0 / N;
   mixed_set_rng(a, desc->seed, desc->instance);
   a.chunks = chunks;
   a.paths_per_chunk = ppc;
   a.n_items = n_items;
   a.want_var = desc->want_var ? 1 : 0;
-  a.dup_sum = ctx->L.geom == 1 ? 1 : desc->dup_sum;  // circle layouts sum shared side knots
   a.adaptive_h = desc->adaptive_h ? 1 : 0;
   a.richardson = desc->richardson ? 1 : 0;
   a.h64 = desc->h;
@@ -657,8 +695,6 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   }
   a.mc_knots = (lpt && ctx->lpt_ready) ? ctx->mc_lpt.p : ctx->mc_knots.p + mc0;
   a.item_counter = ctx->counter.p;
-  a.G = ctx->G.p;
-  a.GG = ctx->GG.p;
   a.Bsum = ctx->Bsum.p;
   a.BBsum = ctx->BBsum.p;
   a.stats = ctx->stats.p;
@@ -666,13 +702,18 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   a.item_knot = items ? items->knot : nullptr;
   a.item_p0 = items ? items->p0 : nullptr;
   a.item_p1 = items ? items->p1 : nullptr;
-  a.knot_invN = items ? items->knot_invN : nullptr;
   a.knot_steps = ctx->knot_steps.p;
   a.step_hist = desc->step_histogram ? ctx->step_hist.p : nullptr;
   a.diag = (desc->diagnostics && ctx->diag.n >= (size_t)ctx->L.K * PDDS_DIAG_N) ? ctx->diag.p : nullptr;
   const int threads = cta_threads_for(ctx, desc);
   const size_t base_smem = ctx->mixed_smem * (a.want_var ? 2 : 1) + mixed_queue_smem(threads, a.richardson);
   a.hist_cap = (int)(ctx->mixed_smem / sizeof(float));
+  a.hist_stride = slot_words(ctx, desc);
+  a.var_off = hist_words(ctx);
+  CK(ctx->hist.resize((size_t)std::max<int64_t>(1, n_items * a.hist_stride)));
+  a.hist_out = ctx->hist.p;
+  a.mc_pos = ctx->mc_pos.p;
+  a.mc0 = mc0;
   const int mk = mixed_kind(P);
   const size_t smem = base_smem + (mk == PK_LUT ? lut_stage(ctx, P, base_smem, threads, &a.lut_nodes) : 0);
   if (smem > 200 * 1024) return fail(ctx, PDDS_ERR_INVALID, "exit histograms exceed shared memory; lower bins_per_gap");
@@ -693,6 +734,44 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
       ++*launches;
       ctx->lpt_ready = true;
     }
+    ContractArgs c{};
+    c.L = ctx->dl;
+    c.hist = ctx->hist.p;
+    c.stride = a.hist_stride;
+    c.var_off = a.var_off;
+    c.chunks = chunks;
+    c.n_rows = mc_n;
+    c.rows = ctx->mc_knots.p + mc0;
+    int max_cnt = chunks;
+    if (items) {  // a row per run of items of one knot, in hand-out order
+      std::vector<std::array<int, 3>> run;  // knot, first slot, slots
+      max_cnt = 1;
+      for (int i = 0; i < items->n; i++) {
+        if (run.empty() || run.back()[0] != items->host[i]) run.push_back({items->host[i], i, 0});
+        max_cnt = std::max(max_cnt, ++run.back()[2]);
+      }
+      std::vector<int> pos(ctx->L.K, 0);
+      for (int m = 0; m < ctx->n_mc; m++) pos[ctx->mc_host[m]] = m;
+      std::stable_sort(run.begin(), run.end(),
+                       [&](const std::array<int, 3>& u, const std::array<int, 3>& v) { return pos[u[0]] < pos[v[0]]; });
+      const size_t nr = run.size();
+      std::vector<int> rows(3 * nr);
+      for (size_t r = 0; r < nr; r++)
+        for (int q = 0; q < 3; q++) rows[q * nr + r] = run[r][q];
+      CK(ctx->item_rows.upload(rows, s));
+      c.n_rows = (int)nr;
+      c.rows = ctx->item_rows.p;
+      c.row_slot = ctx->item_rows.p + nr;
+      c.row_cnt = ctx->item_rows.p + 2 * nr;
+    }
+    c.inv_N = 1.0 / N;
+    c.knot_invN = items ? items->knot_invN : nullptr;
+    c.dup_sum = ctx->L.geom == 1 ? 1 : desc->dup_sum;  // circle layouts sum shared side knots
+    c.G = ctx->G.p;
+    c.GG = desc->want_var ? ctx->GG.p : nullptr;
+    c.err_flags = ctx->errf.p;
+    CK(launch_contract(c, ctx->mixed_smem ? (int)a.hist_stride : 0, ctx->max_n, ctx->max_nbins, max_cnt,
+                       ctx->num_sms, launches, s));
   }
   return PDDS_OK;
 }
@@ -754,7 +833,7 @@ pdds_status adaptive_continue(pdds_ctx* ctx, const pdds_estimate_desc* desc, con
     CK(ctx->item_knot.upload(ik, s));
     CK(ctx->item_p0.upload(ip0, s));
     CK(ctx->item_p1.upload(ip1, s));
-    ItemList items{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), ctx->knot_invN.p};
+    ItemList items{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), ctx->knot_invN.p, ik.data()};
     pdds_estimate_desc dc = *desc;  // the continuation's block size, when the autotuner timed one
     if (dc.cta_threads == 0 && tuned_for(ctx, desc) && ctx->tune_cont_threads > 0)
       dc.cta_threads = ctx->tune_cont_threads;
@@ -762,6 +841,16 @@ pdds_status adaptive_continue(pdds_ctx* ctx, const pdds_estimate_desc* desc, con
     if (st != PDDS_OK) return st;
   }
   return PDDS_OK;
+}
+
+size_t mixed_hist_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int mc_n) {
+  int chunks = 1, ppc = 1;
+  item_split(ctx, desc->npaths, &chunks, &ppc, tuned_for(ctx, desc) ? ctx->tune_ppc : 0, cta_threads_for(ctx, desc),
+             mc_n);
+  const int64_t slots = max_slots(ctx, desc);
+  int64_t n = (int64_t)mc_n * chunks;
+  if (n > slots) n = std::max<int64_t>(slots, chunks);
+  return (size_t)(n * slot_words(ctx, desc));
 }
 
 pdds_status enqueue_mixed(pdds_ctx* ctx, const pdds_estimate_desc* desc, int* launches, int mc0, int mc_n,
@@ -849,7 +938,7 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     for (auto* b : d64) b->recycle();
     DBuf<int>* di[] = {&ctx->knot_stencil, &ctx->st_side, &ctx->st_glob, &ctx->map_pos, &ctx->sd_n,
                        &ctx->sd_orient, &ctx->sd_shape, &ctx->side_knot, &ctx->sh_n, &ctx->sh_nbins,
-                       &ctx->col, &ctx->mc_knots, &ctx->bnd_knots, &ctx->counter, &ctx->rside,
+                       &ctx->col, &ctx->mc_knots, &ctx->mc_pos, &ctx->bnd_knots, &ctx->counter, &ctx->rside,
                        &ctx->rsl, &ctx->rss, &ctx->rbf_piv};
     for (auto* b : di) b->recycle();
     DBuf<int64_t>* dl[] = {&ctx->row_ptr, &ctx->st_map_off, &ctx->sd_knot_off, &ctx->sh_tab_off,
@@ -897,6 +986,8 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     ctx->sub_iters.recycle();
     ctx->ugrid.recycle();
     ctx->item_knot.recycle();
+    ctx->item_rows.recycle();
+    ctx->hist.recycle();
     ctx->item_p0.recycle();
     ctx->item_p1.recycle();
     ctx->knot_scale.recycle();
@@ -1469,7 +1560,7 @@ pdds_status pdds_autotune(pdds_ctx* ctx, const pdds_estimate_desc* desc, int32_t
     CK(ctx->item_knot.upload(ik, s));
     CK(ctx->item_p0.upload(ip0, s));
     CK(ctx->item_p1.upload(ip1, s));
-    ItemList items{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), nullptr};
+    ItemList items{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), nullptr, ik.data()};
     float best = 1e30f;
     for (int rep = 0; rep < 2; rep++) {
       ctx->force_bps = bps;
@@ -1529,7 +1620,7 @@ pdds_status pdds_autotune(pdds_ctx* ctx, const pdds_estimate_desc* desc, int32_t
       CK(ctx->item_knot.upload(ik, s));
       CK(ctx->item_p0.upload(ip0, s));
       CK(ctx->item_p1.upload(ip1, s));
-      ItemList items{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), ctx->knot_invN.p};
+      ItemList items{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), ctx->knot_invN.p, ik.data()};
       pdds_estimate_desc dc = d;
       dc.cta_threads = threads;
       CK(cudaEventRecord(ctx->ev0, s));

@@ -133,7 +133,7 @@ struct pdds_ctx {
   // device layout
   DBuf<double> kx, ky, st_rect, sd_c, sd_origin, side_px, side_py, sh_c, sh_R, sh_lo, sh_delta, sh_t, ipsi;
   DBuf<int> knot_stencil, st_side, st_glob, map_pos, sd_n, sd_orient, sd_shape, side_knot, sh_n,
-      sh_nbins, col, mc_knots, bnd_knots;
+      sh_nbins, col, mc_knots, mc_pos, bnd_knots;
   DBuf<double> rbf_lu, rbf_uinv;  // factorisation scratch (ipsi and sh_t layouts)
   DBuf<int64_t> st_col_off;       // stencils' column lists, expanded into col on the device
   DBuf<int> st_cols;
@@ -148,7 +148,11 @@ struct pdds_ctx {
   std::vector<int> mc_host;  // knots with paths, in hand-out order (the device mc_knots)
   size_t mixed_smem = 0;
   int fp64_nall = 0;              // side knots of the largest stencil
-  int max_nbins = 0;
+  int max_n = 0, max_nbins = 0;   // of the shapes
+  // exit histograms of a MIXED launch's work items, and an item list's rows
+  // (knot, first slot, slots)
+  DBuf<float> hist;
+  DBuf<int> item_rows;
   // results and scratch
   DBuf<double> G, GG, B, BB, Bsum, BBsum;
   DBuf<unsigned long long> stats;
@@ -248,6 +252,8 @@ pdds_status check_err_flags(pdds_ctx* ctx);
 // end); prefix: also the factorisation, zeroing and boundary knots.
 pdds_status enqueue_mixed(pdds_ctx* ctx, const pdds_estimate_desc* desc, int* launches, int mc0 = 0,
                           int mc_n = -1, bool prefix = true);
+// Words of exit histograms that enqueue_mixed needs for mc_n knots.
+size_t mixed_hist_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int mc_n);
 // Destroys the captured batch graph (its kernels hold buffer addresses).
 void drop_graph(pdds_ctx* ctx);
 // Forgets the autotuned launch shape (it was timed on the previous layout).

@@ -33,8 +33,6 @@ struct ItemSide {
   int glob;
   float base;
   float inv_delta;
-  int64_t tab_off;
-  int64_t map_off;
 };
 
 // Kinds whose Y changes along a path (a reaction term, or Robin local time).
@@ -261,7 +259,6 @@ k_paths_mixed(const MixedArgs a) {
         is.glob = L.st_glob[4 * st + d];
         if (sd < 0) {
           is.n = 0; is.nbins = 0; is.hist_off = 0; is.orient = 0; is.base = 0.f; is.inv_delta = 0.f;
-          is.tab_off = 0; is.map_off = 0;
         } else {
           const int sh = L.sd_shape[sd];
           is.n = L.sd_n[sd];
@@ -276,16 +273,9 @@ k_paths_mixed(const MixedArgs a) {
           }
           is.base = (float)(origin + L.sh_lo[sh] - delta);
           is.inv_delta = (float)(1.0 / delta);
-          is.tab_off = L.sh_tab_off[sh];
           off += is.nbins;
         }
         s_side[d] = is;
-      }
-      // side-knot -> row position maps, in side order
-      int64_t moff = L.st_map_off[st];
-      for (int d = 0; d < 4; d++) {
-        s_side[d].map_off = moff;
-        moff += s_side[d].n;
       }
       s_hist_len = off;
     }
@@ -926,35 +916,14 @@ k_paths_mixed(const MixedArgs a) {
     }
     if (a.step_hist && tid < 32 && s_sth[tid]) atomicAdd(a.step_hist + tid, (unsigned long long)s_sth[tid]);
     if constexpr (DIAG) diag_flush(s_dg, a.diag + (int64_t)knot * PDDS_DIAG_N, tid);
-    // ------------------------------------------------------------ contract G
-    const int64_t row0 = L.row_ptr[knot];
-    const double invN = a.knot_invN ? a.knot_invN[knot] : a.inv_N;
-    const int n_all = s_side[0].n + s_side[1].n + s_side[2].n + s_side[3].n;
-    for (int pr = tid; pr < n_all; pr += nthr) {
-      int d = 0, i = pr;
-      while (i >= s_side[d].n) { i -= s_side[d].n; ++d; }
-      const ItemSide& is = s_side[d];
-      const int64_t m = is.map_off + i;
-      if (!a.dup_sum && !L.map_owner[m]) continue;
-      const float* tab = L.tab + is.tab_off + i;
-      const float* hs = hist + is.hist_off;
-      const float* hs2 = hist2 + is.hist_off;
-      double acc = 0.0, acc2 = 0.0;
-      for (int b0 = 0; b0 < is.nbins; b0 += 64) {
-        const int b1 = min(is.nbins, b0 + 64);
-        float part = 0.f, part2 = 0.f;
-        for (int q = b0; q < b1; q++) {
-          const float hv = __ldg(tab + (int64_t)q * is.n);
-          part = fmaf(hs[q], hv, part);
-          if (a.want_var) part2 = fmaf(hs2[q], hv * hv, part2);
-        }
-        acc += (double)part;
-        acc2 += (double)part2;
-      }
-      const int64_t e = row0 + L.map_pos[m];
-      if (!idx_ok(e - row0, L.row_ptr[knot + 1] - row0, a.err_flags)) continue;
-      atomicAdd(a.G + e, -acc * invN);
-      if (a.want_var) atomicAdd(a.GG + e, acc2 * invN);
+    // ------------------------------------------------------------ histograms out
+    // k_contract turns them into the knot's row of G
+    float* out = a.hist_out + a.hist_stride *
+                                  (a.item_knot ? (int64_t)item
+                                               : (int64_t)(a.mc_pos[knot] - a.mc0) * a.chunks + item % a.chunks);
+    for (int i = tid; i < hist_len; i += nthr) {
+      __stcs(out + i, hist[i]);
+      if (a.want_var) __stcs(out + a.var_off + i, hist2[i]);
     }
     __syncthreads();
   }

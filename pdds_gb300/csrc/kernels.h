@@ -72,40 +72,62 @@ struct MixedArgs {
   ProblemDev P;
   int N;                 // paths per knot
   float h, sqrth;
-  double inv_N;
   // Philox-4x32-10 round keys of the seed (k0 + r W0, k1 + r W1 for rounds
   // r = 0..9, set by mixed_set_rng): kernel parameters, so every round's key
   // is an operand of its XOR instead of a key-schedule addition per call
   uint32_t rk[20];
   uint32_t instance;
   int chunks, paths_per_chunk, n_items;
-  int want_var, dup_sum;
+  int want_var;
   int adaptive_h;
   int richardson;        // 1: common-random-number Richardson pair (h/2, h)
   double h64;            // h in FP64 (for the adaptive step)
   long long max_steps;
   const int* mc_knots;   // knots that need paths, in hand-out order
   int hist_cap;          // words reserved for one exit histogram
+  // the items' histograms: item i of a list at slot i, chunk c of a knot at
+  // slot (mc_pos[knot] - mc0) chunks + c, hist_stride words each, the Y^2
+  // histogram var_off words after the first
+  float* hist_out;
+  int64_t hist_stride;
+  int var_off;
+  const int* mc_pos;     // position of each knot in the hand-out order
+  int mc0;
   int lut_nodes;         // table nodes that can be staged in shared memory (PK_LUT)
   int* item_counter;
-  double* G;             // [nnz] accumulates -sum Y H / N
-  double* GG;            // [nnz] accumulates sum (Y H)^2 / N
   double* Bsum;          // [K]
   double* BBsum;         // [K]
   unsigned long long* stats;  // [0] steps [1] unused [2] global exits [3] stencil exits
   unsigned* err_flags;
-  // optional explicit items (knot, paths [p0, p1)) instead of n_mc x chunks,
-  // and per-knot 1/N_k instead of inv_N (variance-adaptive paths)
+  // optional explicit items (knot, paths [p0, p1)) instead of n_mc x chunks
   const int* item_knot;
   const int* item_p0;
   const int* item_p1;
-  const double* knot_invN;
   unsigned long long* knot_steps;  // optional: path steps per knot (both levels)
   // optional [32]: paths (each level of a Richardson pair counts) by their
   // steps, bin b = steps in [2^b, 2^(b+1))
   unsigned long long* step_hist;
   // optional [K][PDDS_DIAG_N]: the reduction's diagnostic sums per knot
   double* diag;
+};
+
+// Rows of G from the path kernel's histograms (k_contract.cu).
+struct ContractArgs {
+  DevLayout L;
+  float* hist;           // slots of `stride` words; a row's slots are summed into its first
+  int64_t stride;
+  int var_off;           // words from a slot's histogram to its Y^2 histogram
+  int n_rows;
+  const int* rows;       // knots, in hand-out order
+  int chunks;            // slots per row, unless
+  const int* row_slot;   // each row has its own first slot
+  const int* row_cnt;    // and number of slots
+  double inv_N;
+  const double* knot_invN;  // optional: 1/N_k instead of inv_N (variance-adaptive paths)
+  int dup_sum;
+  double* G;             // [nnz] accumulates -sum Y H / N
+  double* GG;            // [nnz] accumulates sum (Y H)^2 / N; null without variances
+  unsigned* err_flags;
 };
 
 struct Fp64Args {
@@ -186,6 +208,9 @@ inline int mixed_kind(const ProblemDev& P) { return P.kind == PK_LUT && P.lut.te
 // smem: mixed_queue_smem(threads, richardson) + the exit histograms
 cudaError_t launch_paths_mixed(const MixedArgs& a, int kind, int grid, int threads, size_t smem, cudaStream_t s);
 size_t mixed_queue_smem(int threads, int richardson);
+// words: of a slot; max_n, max_nbins: of the layout's shapes; max_cnt: slots of a row
+cudaError_t launch_contract(const ContractArgs& a, int words, int max_n, int max_nbins, int max_cnt, int num_sms,
+                            int* launches, cudaStream_t s);
 // knots mc[n] reordered heaviest first by steps[knot] (quarter-octave groups)
 cudaError_t launch_lpt_order(const int* mc, int n, const unsigned long long* steps, int* out, cudaStream_t s);
 // Sets the Philox key schedule (rk) of `seed` and the instance word.

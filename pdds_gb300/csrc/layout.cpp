@@ -129,7 +129,7 @@ void set_shape_bins(HostLayout& L, int bps) {
     const int inner = (int)std::ceil((sh.hi - sh.lo) / sh.delta - 1e-9);
     sh.nbins = inner + 4;  // grid covers [lo - delta, hi + 2 delta]
     sh.tab_off = tab;
-    tab += (int64_t)sh.nbins * sh.n;
+    tab += ((int64_t)sh.nbins * sh.n + 3) & ~int64_t(3);  // 16-byte copies of the table
   }
 }
 
