@@ -19,13 +19,14 @@
 // knots 0.433 -> 0.404).
 //
 // Rounding: before, each work item had FP32 sums of 64 products, added up in
-// FP64.  Here a knot's items are added first, in two floats rounded once, so
-// the products' rounding no longer averages over the items: FP32 sums are
-// 8 products long (4 from 5 items per knot on) and are added up in two floats
-// (TwoSum, 48 bits; FP64 issues at 1/64 of the rate).  Against exact sums of
-// the same histograms, G is off by (rms, before and now) 4.0e-8 and 2.0e-8
-// with 11 items per knot, 6.5e-8 and 3.4e-8 with 4, 1.3e-7 and 4.3e-8 with 1;
-// sums of 16 products: 5.6e-8 with 11 items.  The time is the same for 8.
+// FP64.  With one item per knot it is the same here, the 64-product sums added
+// in two floats (TwoSum, 48 bits; FP64 issues at 1/64 of the rate).  Several
+// items of a knot are added first, in two floats rounded once, so the
+// products' rounding no longer averages over the items: the FP32 sums are
+// then 8 products long, 4 from 5 items on.  Against exact sums of the same
+// histograms, G is off by (rms, before and now) 4.0e-8 and 2.0e-8 with 11
+// items per knot, 6.5e-8 and 3.4e-8 with 4 (with sums of 16 products 5.6e-8
+// and 5.8e-8); the time is the same.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -192,16 +193,26 @@ __device__ __forceinline__ void contract_columns(const ContractArgs& a, const Ro
           }
         }
     };
-    int q = 0;
+    if constexpr (SUM > CT_BINS) {
+      if (qn == CT_BINS) {
+#pragma unroll 8
+        for (int q = 0; q < CT_BINS; q++) bin(q);
+      } else {
+        for (int q = 0; q < qn; q++) bin(q);
+      }
+      if ((st + 1) % (SUM / CT_BINS) == 0 || st == st1 - 1) flush();
+    } else {
+      int q = 0;
 #pragma unroll 1
-    for (; q + SUM <= qn; q += SUM) {
+      for (; q + SUM <= qn; q += SUM) {
 #pragma unroll
-      for (int k = 0; k < SUM; k++) bin(q + k);
-      flush();
-    }
-    if (q < qn) {
-      for (; q < qn; q++) bin(q);
-      flush();
+        for (int k = 0; k < SUM; k++) bin(q + k);
+        flush();
+      }
+      if (q < qn) {
+        for (; q < qn; q++) bin(q);
+        flush();
+      }
     }
   }
   __syncthreads();  // the ring is free
@@ -269,8 +280,9 @@ __global__ void __launch_bounds__(Tile<VAR>::THREADS, VAR ? 2 : 3) k_contract(co
     const int first = __ffs(todo) - 1;
     const unsigned rows = __ballot_sync(FULLM, mine == s_row[first].tab) & todo;
     const int n = s_row[first].n, stages = (s_row[first].nbins + CT_BINS - 1) / CT_BINS;
-    const int st0 = (int)((int64_t)stages * blockIdx.z / gridDim.z);
-    const int st1 = (int)((int64_t)stages * (blockIdx.z + 1) / gridDim.z);
+    const int pair = (stages + 1) / 2;  // the split leaves every 64 bins together
+    const int st0 = 2 * (int)((int64_t)pair * blockIdx.z / gridDim.z);
+    const int st1 = min(stages, 2 * (int)((int64_t)pair * (blockIdx.z + 1) / gridDim.z));
     if (st0 < st1)
       for (int c0 = 0; c0 < n; c0 += 32 * Tile<VAR>::NJ) {
         const int left = n - c0;
@@ -321,10 +333,14 @@ cudaError_t launch_contract(const ContractArgs& a, int words, int max_n, int max
     ++*launches;
     return cudaGetLastError();
   };
-  const bool many = max_cnt > 4;
+  // FP32 sums as long as the rounding allows (see above)
   if (a.GG)
-    return run(many ? k_contract<true, 4> : k_contract<true, 8>, Tile<true>::THREADS, Tile<true>::A_WORDS);
-  return run(many ? k_contract<false, 4> : k_contract<false, 8>, Tile<false>::THREADS, Tile<false>::A_WORDS);
+    return max_cnt > 4   ? run(k_contract<true, 4>, Tile<true>::THREADS, Tile<true>::A_WORDS)
+           : max_cnt > 1 ? run(k_contract<true, 8>, Tile<true>::THREADS, Tile<true>::A_WORDS)
+                         : run(k_contract<true, 64>, Tile<true>::THREADS, Tile<true>::A_WORDS);
+  return max_cnt > 4   ? run(k_contract<false, 4>, Tile<false>::THREADS, Tile<false>::A_WORDS)
+         : max_cnt > 1 ? run(k_contract<false, 8>, Tile<false>::THREADS, Tile<false>::A_WORDS)
+                       : run(k_contract<false, 64>, Tile<false>::THREADS, Tile<false>::A_WORDS);
 }
 
 }  // namespace pdds
