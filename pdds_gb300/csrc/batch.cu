@@ -26,12 +26,52 @@ int batch_waves(const pdds_ctx* ctx, const pdds_batch_run_desc* d) {
   return std::max(1, std::min(ctx->n_inst, d->waves > 0 ? d->waves : 16));
 }
 
+// Splits of the last group's systems [i0, n_inst) for the solve with the
+// system on chip (k_resident.cu), which takes all SMs: nothing else is left
+// to run beside that group's solves, while the cluster kernel (16 SMs per
+// system) leaves most of the chip idle.  A batch of 24 whose last group has
+// 14,952 and 19,005 rows ends 9.6 ms earlier (147.9 -> 138.4 ms).  Not for
+// many systems at once, which fill the chip: one system takes a third (237
+// rows) to a seventh (19,005 rows) of the cluster kernel's time, but one
+// follows the other, and the cluster kernel runs num_sms / cluster at a time.
+// The classical form and systems that do not fit keep the cluster.
+constexpr int TAIL_GAIN = 3;
+const std::vector<ResidentPlan>& batch_tail(pdds_ctx* ctx, const pdds_batch_run_desc* d, int cluster, int i0, int m) {
+  pdds_ctx::BatchTail& t = ctx->batch_tail;
+  if (!t.ready || t.i0 != i0 || t.m != m) {
+    t.plans.clear();
+    t.i0 = i0;
+    t.m = m;
+    t.ready = true;
+    const int n = ctx->n_inst - i0;
+    const int rounds = (n * cluster + ctx->num_sms - 1) / std::max(ctx->num_sms, 1);
+    for (int i = i0; i < ctx->n_inst && n <= TAIL_GAIN * rounds; i++) {
+      const int k0 = ctx->inst_k0[i];
+      const ResidentRows rows{ctx->inst_k0[i + 1] - k0, ctx->L.row_ptr.data() + k0, ctx->L.knot_stencil.data() + k0};
+      t.plans.push_back(resident_plan(rows, RESIDENT_GMRES, m, 0));
+      if (t.plans.back().ctas < 1) {
+        t.plans.clear();
+        break;
+      }
+    }
+  }
+  static const std::vector<ResidentPlan> none;
+  return d->solve.gmres_form == PDDS_GMRES_PIPELINED ? t.plans : none;
+}
+
+// First instance of the last group.
+int tail_first(const pdds_ctx* ctx, const pdds_batch_run_desc* d) {
+  const int W = batch_waves(ctx, d);
+  return (int)((int64_t)ctx->n_inst * (W - 1) / W);
+}
+
 // The whole batch step, without host synchronisation.  The stream runs the
 // factorisation, zeroing and boundary knots, then the instances in W
 // consecutive groups (a path-kernel launch and the finalisation per group);
 // the solve stream, once a group's finalisation is done, copies its G rows
 // to FP32 and runs the cluster GMRES of its systems while the next group's
-// paths run.  The last solve joins the stream again.
+// paths run.  The last group's systems are solved on the whole chip, one
+// after another (batch_tail); the last solve joins the stream again.
 pdds_status enqueue_batch(pdds_ctx* ctx, const pdds_batch_run_desc* d, int cluster, int* launches) {
   cudaStream_t s = ctx->stream, s2 = ctx->solve_stream;
   const int n = ctx->n_inst;
@@ -64,6 +104,36 @@ pdds_status enqueue_batch(pdds_ctx* ctx, const pdds_batch_run_desc* d, int clust
     if (st != PDDS_OK) return st;
     CK(cudaEventRecord(ctx->wave_ev[w], s));
     CK(cudaStreamWaitEvent(s2, ctx->wave_ev[w], 0));
+    if (w == W - 1) {
+      const std::vector<ResidentPlan>& plans = batch_tail(ctx, d, cluster, i0, a.m);
+      for (size_t q = 0; q < plans.size(); q++) {
+        const int i = i0 + (int)q, k0 = ctx->inst_k0[i];
+        ResidentArgs r{};
+        r.K = ctx->inst_k0[i + 1] - k0;
+        r.row_ptr = ctx->row_ptr.p + k0;
+        r.knot_stencil = ctx->knot_stencil.p + k0;
+        r.st_off = ctx->st_col_off.p;
+        r.st_cols = ctx->st_cols.p;
+        r.col0 = k0;
+        r.val64 = ctx->G.p;
+        r.rest = ctx->sval32.p;
+        r.b = ctx->B.p + k0;
+        r.x = ctx->su.p + k0;
+        r.m = a.m;
+        r.max_iter = a.max_iter;
+        r.max_refine = a.max_refine;
+        r.tol = a.tol;
+        r.inner_tol = a.inner_tol;
+        r.out_iters = ctx->b_iters.p + i;
+        r.out_refines = ctx->b_refines.p + i;
+        r.out_relres = ctx->b_relres.p + i;
+        r.out_t_end = ctx->b_tend.p + i;
+        r.err_flags = ctx->errf.p;
+        CK(launch_resident(r, plans[q], RESIDENT_GMRES, ctx->sexch.p, s2));
+        ++*launches;
+      }
+      if (!plans.empty()) break;
+    }
     const int64_t e0 = ctx->inst_nnz0[i0], e1 = ctx->inst_nnz0[i1];
     CK(launch_to_f32(ctx->G.p + e0, ctx->sval32.p + e0, e1 - e0, s2));
     ++*launches;
@@ -223,19 +293,21 @@ pdds_status pdds_batch_run(pdds_ctx* ctx, const pdds_batch_run_desc* desc, pdds_
   const int64_t nnz = L.row_ptr[L.K];
   const int m = std::max(2, std::min(desc->solve.restart > 0 ? desc->solve.restart : 30, GMRES_CLUSTER_MAX_M));
   // buffers first: a captured graph holds their addresses
-  const void* before[6] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p, ctx->hist.p};
+  const void* before[7] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p, ctx->hist.p, ctx->sexch.p};
   size_t hw = 1;
   for (int w = 0, W = batch_waves(ctx, desc); w < W; w++) {
     const int i0 = (int)((int64_t)ctx->n_inst * w / W), i1 = (int)((int64_t)ctx->n_inst * (w + 1) / W);
     hw = std::max(hw, mixed_hist_words(ctx, &ed, ctx->inst_mc0[i1] - ctx->inst_mc0[i0]));
   }
   CK(ctx->hist.resize(hw));
+  if (!batch_tail(ctx, desc, cluster, tail_first(ctx, desc), m).empty())
+    CK(ctx->sexch.resize(resident_exchange_bytes(ctx->max_inst_knots)));
   CK(ctx->sV32.resize((size_t)(m + 1) * K));
   if (desc->solve.gmres_form == PDDS_GMRES_PIPELINED) CK(ctx->sZ32.resize((size_t)(m + 1) * K));
   CK(ctx->sval32.resize(std::max<int64_t>(nnz, 1)));
   CK(ctx->sv64.resize(std::max<int64_t>(K, 1) * 6));
   CK(ctx->su.resize(std::max<int64_t>(K, 1)));
-  const void* after[6] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p, ctx->hist.p};
+  const void* after[7] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p, ctx->hist.p, ctx->sexch.p};
   if (std::memcmp(before, after, sizeof(before)) != 0) drop_graph(ctx);
   // the graph is reused while the descriptor, the cluster size and the solve
   // scratch (which pdds_solve_interface may also reallocate) are unchanged;

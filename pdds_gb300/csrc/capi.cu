@@ -267,6 +267,7 @@ pdds_status upload_layout(pdds_ctx* ctx) {
   ctx->ugrid_m = 0;
   ctx->lpt_ready = false;
   ctx->solve_plan[0].ready = ctx->solve_plan[1].ready = false;
+  ctx->batch_tail.ready = false;
   HostLayout& L = ctx->L;
   cudaStream_t s = ctx->stream;
   std::vector<double> st_rect;
@@ -1912,6 +1913,7 @@ pdds_status pdds_solve_interface(pdds_ctx* ctx, const pdds_solve_desc* desc, dou
   CK(cudaEventRecord(ctx->ev0, s));
   if (plan.ctas > 0) {
     CK(ctx->sexch.resize(resident_exchange_bytes(K)));
+    if (plan.rest) CK(ctx->sval32.resize(std::max<int64_t>(nnz, 1)));
     ResidentArgs a{};
     a.K = K;
     a.row_ptr = ctx->row_ptr.p;
@@ -1919,6 +1921,7 @@ pdds_status pdds_solve_interface(pdds_ctx* ctx, const pdds_solve_desc* desc, dou
     a.st_off = ctx->st_col_off.p;
     a.st_cols = ctx->st_cols.p;
     a.val64 = ctx->G.p;
+    a.rest = ctx->sval32.p;
     a.b = ctx->B.p;
     a.x = ctx->su.p;
     a.m = m;

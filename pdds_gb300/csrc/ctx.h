@@ -177,6 +177,13 @@ struct pdds_ctx {
     int m = 0, grid_ctas = 0;
     pdds::ResidentPlan plan;
   } solve_plan[2];
+  // the same for the last group of a batch (batch.cu), one split per system;
+  // no splits: the group's systems run the cluster kernel
+  struct BatchTail {
+    bool ready = false;
+    int i0 = 0, m = 0;
+    std::vector<pdds::ResidentPlan> plans;
+  } batch_tail;
   int solve_m = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   // batch of independent instances (pdds_batch_build): the layout above is

@@ -26,6 +26,9 @@
 //  * FP64 issues at 1/64 of the FP32 rate, one warp instruction per 64 cycles
 //    and scheduler: FP64 scalars are formed by one warp and passed through
 //    shared memory, and sums involve only the warps that hold rows.
+//  * of a larger system the entries that do not fit are read from L2 as FP32
+//    (up to half of a CTA's): 19,005 rows, 6.9 M entries, GMRES(20) 1,665 ->
+//    1,526 us against the kernel that reads values and columns from L2.
 // Measured (median of 5, before -> now): GMRES(20) 237 rows 501 -> 165 us,
 // 741 rows 847 -> 214, 2,205 rows 1,500 -> 365, 3,325 rows 2,780 -> 508,
 // 10,989 rows (120 steps) 1,945 -> 980 us; BiCGSTAB 3,325 rows 2,956 -> 890,
@@ -269,7 +272,7 @@ __device__ Part build_part(const ResidentArgs& a, const Carve& c, unsigned char*
     if (len == 0) continue;
     const int* cols = a.st_cols + a.st_off[a.knot_stencil[r0 + q]];
     for (int i = lane; i < len; i += 32) {
-      const int col = __ldg(cols + i);
+      const int col = __ldg(cols + i) - a.col0;
       if (idx_ok(col, a.K, a.err_flags)) atomicOr(&bits[col >> 5], 1u << (col & 31));
     }
   }
@@ -303,7 +306,7 @@ __device__ Part build_part(const ResidentArgs& a, const Carve& c, unsigned char*
     if (len == 0) continue;
     const int* cols = a.st_cols + a.st_off[a.knot_stencil[r0 + q]];
     for (int i = lane; i < len; i += 32) {
-      const int col = __ldg(cols + i);
+      const int col = __ldg(cols + i) - a.col0;
       if (!idx_ok(col, a.K, a.err_flags)) continue;
       list[at + i] = (unsigned short)(pre[col >> 5] + __popc(bits[col >> 5] & ((1u << (col & 31)) - 1u)));
     }
@@ -381,6 +384,15 @@ __device__ __forceinline__ T seg_sum(const Part& p, int per, const T* out, int q
 
 __device__ __forceinline__ void write_out(const ResidentArgs& a, bool alive, int total, int ref, double relres) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!a.out) {
+      *a.out_iters = total;
+      *a.out_refines = ref;
+      *a.out_relres = alive ? relres : -1.0;
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      *a.out_t_end = t;
+      return;
+    }
     a.out[0] = alive ? relres : -1.0;
     reinterpret_cast<int*>(a.out + 1)[0] = total;
     reinterpret_cast<int*>(a.out + 1)[1] = ref;
@@ -430,9 +442,14 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_resident_gmres(const Resident
       for (int u = 0; u < U; u++) t[u] = e0 + RS_THREADS * u < nn ? __ldg(v64 + e0 + RS_THREADS * u) : 0.0;
 #pragma unroll
       for (int u = 0; u < U; u++)
-        if (e0 + RS_THREADS * u < nn) val[e0 + RS_THREADS * u] = (float)t[u];
+        if (const int e = e0 + RS_THREADS * u; e < nn) {
+          if (e < a.cap_nnz) val[e] = (float)t[u];
+          else a.rest[p.e0 + e] = (float)t[u];
+        }
     }
   }
+  const bool all_here = p.voff[nown] <= a.cap_nnz;
+  const float* rest = all_here ? nullptr : a.rest + p.e0;
   unsigned seqp = 0, seqt = 0, seqx = 0;  // publications of partials, of Krylov vectors, of x
   bool alive = true;                      // false once a wait ran out: the CTA winds down
   auto all_ok = [&](bool ok) -> bool {    // CTA barrier; later waits do not wait again
@@ -622,8 +639,14 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_resident_gmres(const Resident
             s_flag = (fabsf(gj) <= (float)a.inner_tol || !(hn > 0.f)) ? 1 : 0;
           }
         }
-        if (j < m)
-          products<float>(p, per, xf, warp, j > 0 ? RS_WARPS - 1 : RS_WARPS, lane, [&](int e) { return val[e]; }, w);
+        if (j < m) {
+          const int warps = j > 0 ? RS_WARPS - 1 : RS_WARPS;
+          if (all_here)
+            products<float>(p, per, xf, warp, warps, lane, [&](int e) { return val[e]; }, w);
+          else
+            products<float>(p, per, xf, warp, warps, lane,
+                            [&](int e) { return e < a.cap_nnz ? val[e] : rest[e]; }, w);
+        }
         __syncthreads();
         if (j > 0) {
           jdim = j;
@@ -907,7 +930,7 @@ constexpr size_t RES_SMEM_CAP = 216 * 1024;  // dynamic; the kernels' static sha
 // counts as ROW_COST more), and what the largest CTA needs.
 constexpr int ROW_COST = 32;
 void plan_rows(const ResidentRows& rows, int ctas, ResidentPlan& p) {
-  const int64_t all = rows.row_ptr[rows.K] + (int64_t)ROW_COST * rows.K;
+  const int64_t e0 = rows.row_ptr[0], all = rows.row_ptr[rows.K] - e0 + (int64_t)ROW_COST * rows.K;
   p.ctas = ctas;
   p.per = p.cap_nnz = p.cap_list = p.cap_loc = 0;
   int r = 0;
@@ -916,7 +939,7 @@ void plan_rows(const ResidentRows& rows, int ctas, ResidentPlan& p) {
     const int64_t upto = all * (c + 1) / ctas;
     int64_t list = 0, nnz = 0;
     const int first = r;
-    while (r < rows.K && (c == ctas - 1 || rows.row_ptr[r + 1] + (int64_t)ROW_COST * (r + 1) <= upto)) {
+    while (r < rows.K && (c == ctas - 1 || rows.row_ptr[r + 1] - e0 + (int64_t)ROW_COST * (r + 1) <= upto)) {
       const int64_t len = rows.row_ptr[r + 1] - rows.row_ptr[r];
       if (r == first || rows.knot_stencil[r] != rows.knot_stencil[r - 1] ||
           len != rows.row_ptr[r] - rows.row_ptr[r - 1])
@@ -941,6 +964,14 @@ bool plan_fits(const ResidentRows& rows, int method, int m, ResidentPlan& p) {
     // the 12x12/n43 entries on chip measured no faster)
     p.cap_nnz = 0;
     p.smem = carve(method, rows.K, m, p.per, 0, p.cap_list, p.cap_loc).total;
+  } else if (p.smem > RES_SMEM_CAP) {
+    // what does not fit is read from L2, as long as it is the smaller part
+    const size_t over = p.smem - RES_SMEM_CAP;
+    const int keep = p.cap_nnz - (int)((over + 15) / 16 * 4) - 4;
+    if (2 * (int64_t)keep < p.cap_nnz) return false;
+    p.cap_nnz = keep & ~3;
+    p.rest = true;
+    p.smem = carve(method, rows.K, m, p.per, p.cap_nnz, p.cap_list, p.cap_loc).total;
   }
   return p.smem <= RES_SMEM_CAP;
 }

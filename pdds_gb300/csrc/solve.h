@@ -93,6 +93,7 @@ struct ResidentPlan {
   int row0[RESIDENT_MAX_CTAS + 1] = {0};
   int per = 0;
   int cap_nnz = 0, cap_list = 0, cap_loc = 0;
+  bool rest = false;  // GMRES: a CTA's entries beyond cap_nnz are read from L2
   size_t smem = 0;
 };
 struct ResidentArgs {
@@ -102,11 +103,17 @@ struct ResidentArgs {
   const int64_t* st_off;
   const int* st_cols;
   const double* val64;
+  float* rest;               // FP32 entries that do not fit on chip, at val64's offsets (with ResidentPlan::rest)
   const double* b;
   double* x;
   int m, max_iter, max_refine;
   double tol, inner_tol;
-  double* out;               // relative residual, then (iterations, refinements) as two ints
+  int col0;                  // subtracted from the columns (a system of a batch: its first row)
+  double* out;               // relative residual, then (iterations, refinements) as two ints; null: the next four
+  int* out_iters;
+  int* out_refines;
+  double* out_relres;
+  unsigned long long* out_t_end;  // %globaltimer at the end (ns)
   unsigned* err_flags;
   unsigned spin_limit;       // polls before a wait gives up (0: the default, about a second)
   // filled in by launch_resident
@@ -116,7 +123,7 @@ struct ResidentArgs {
   ulonglong2* pub;           // 2 K: tagged FP64 vectors (x; r and v)
   unsigned long long* T;     // 2 K: tagged Krylov vectors
 };
-// Host rows of a layout: row k has row_ptr[k + 1] - row_ptr[k] entries, its
+// Host rows of a system: row k has row_ptr[k + 1] - row_ptr[k] entries, its
 // stencil's columns (none on the boundary).
 struct ResidentRows {
   int K;
