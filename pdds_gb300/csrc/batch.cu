@@ -100,7 +100,7 @@ pdds_status enqueue_batch(pdds_ctx* ctx, const pdds_batch_run_desc* d, int clust
   for (int w = 0; w < W; w++) {
     const int i0 = (int)((int64_t)n * w / W), i1 = (int)((int64_t)n * (w + 1) / W);
     const int m0 = ctx->inst_mc0[i0], m1 = ctx->inst_mc0[i1];
-    st = enqueue_mixed(ctx, &d->estimate, launches, m0, m1 - m0, false);
+    st = enqueue_mixed(ctx, &d->estimate, launches, m0, m1 - m0, false, ctx->mc_lpt.p + m0);
     if (st != PDDS_OK) return st;
     CK(cudaEventRecord(ctx->wave_ev[w], s));
     CK(cudaStreamWaitEvent(s2, ctx->wave_ev[w], 0));
@@ -295,9 +295,15 @@ pdds_status pdds_batch_run(pdds_ctx* ctx, const pdds_batch_run_desc* desc, pdds_
   // buffers first: a captured graph holds their addresses
   const void* before[7] = {ctx->sV32.p, ctx->sval32.p, ctx->sv64.p, ctx->su.p, ctx->sZ32.p, ctx->hist.p, ctx->sexch.p};
   size_t hw = 1;
+  std::vector<int> first(1, 0);  // hand-out positions of the groups
   for (int w = 0, W = batch_waves(ctx, desc); w < W; w++) {
     const int i0 = (int)((int64_t)ctx->n_inst * w / W), i1 = (int)((int64_t)ctx->n_inst * (w + 1) / W);
     hw = std::max(hw, mixed_hist_words(ctx, &ed, ctx->inst_mc0[i1] - ctx->inst_mc0[i0]));
+    first.push_back(ctx->inst_mc0[i1]);
+  }
+  {
+    pdds_status st = order_groups(ctx, &ed, first);
+    if (st != PDDS_OK) return st;
   }
   CK(ctx->hist.resize(hw));
   if (!batch_tail(ctx, desc, cluster, tail_first(ctx, desc), m).empty())

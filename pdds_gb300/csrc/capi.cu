@@ -268,6 +268,7 @@ pdds_status upload_layout(pdds_ctx* ctx) {
   ctx->lpt_ready = false;
   ctx->solve_plan[0].ready = ctx->solve_plan[1].ready = false;
   ctx->batch_tail.ready = false;
+  ctx->lpt_groups.clear();
   HostLayout& L = ctx->L;
   cudaStream_t s = ctx->stream;
   std::vector<double> st_rect;
@@ -584,9 +585,42 @@ size_t lut_stage(const pdds_ctx* ctx, const ProblemDev& P, size_t base_smem, int
   return *nodes > 0 ? (size_t)*nodes * 2 * sizeof(float4) + 16 : 0;
 }
 
+// Knots at the hand-out positions [mc0, mc0 + mc_n), heaviest first by a
+// geometric estimate: E[steps] ~ tau / h_k, where tau = tx ty / (tx + ty)
+// combines the expected exit times a (w - a) / 2 across the stencil in x and
+// in y, and h_k is the knot's step (the adaptive one shrinks with the
+// distance d to the nearest side).  It ranks the heavy knots (the cross knots
+// of large stencils and knots close to a side) near the top.
+std::vector<int> geometric_order(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int mc0, int mc_n) {
+  const HostLayout& L = ctx->L;
+  std::vector<std::pair<double, int>> cost;
+  cost.reserve(mc_n);
+  int inst = 0;
+  for (int m = mc0; m < mc0 + mc_n; m++) {
+    const int v = ctx->mc_host[m];
+    const double* r = L.stencils[L.knot_stencil[v]].rect;
+    const double ax = L.kx[v] - r[0], bx = r[2] - L.kx[v], ay = L.ky[v] - r[1], by = r[3] - L.ky[v];
+    const double tx = 0.5 * std::max(ax * bx, 0.0), ty = 0.5 * std::max(ay * by, 0.0);
+    const double tau = tx + ty > 0.0 ? tx * ty / (tx + ty) : 0.0;
+    const double d = std::min(std::min(ax, bx), std::min(ay, by));
+    double hk = desc->h;
+    if (ctx->is_batch) {
+      while (inst + 1 < ctx->n_inst && v >= ctx->inst_k0[inst + 1]) inst++;
+      if (ctx->inst_hv[inst] > 0.0) hk = ctx->inst_hv[inst];
+    }
+    if (desc->adaptive_h && d > 1e-4) hk = std::min(hk, std::pow(d / (2.0 * 0.5826 * 1.4142135623730951), 2.0));
+    cost.push_back({-tau / hk, v});
+  }
+  std::stable_sort(cost.begin(), cost.end());
+  std::vector<int> ord;
+  ord.reserve(cost.size());
+  for (auto& c : cost) ord.push_back(c.second);
+  return ord;
+}
+
 pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, const ProblemDev& P, int chunks,
                                 int ppc, int* launches, const ItemList* items = nullptr, int mc0 = 0,
-                                int mc_n = -1) {
+                                int mc_n = -1, const int* order = nullptr) {
   cudaStream_t s = ctx->stream;
   if (mc_n < 0) mc_n = ctx->n_mc;
   // more work items than histogram slots: one launch after another
@@ -669,32 +703,11 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   // before the first one by a geometric estimate of the steps per path
   const bool lpt = !items && !ctx->is_batch && !desc->plain_launch && mc0 == 0 && mc_n == ctx->n_mc;
   if (lpt && !ctx->lpt_ready && ctx->L.geom == 0) {
-    // E[steps] ~ tau / h_k: tau = tx ty / (tx + ty) combines the expected
-    // exit times a (w - a) / 2 across the stencil in x and in y, h_k is the
-    // knot's step (the adaptive one shrinks with the distance d to the
-    // nearest side).  It ranks the heavy knots (the cross knots of large
-    // stencils and knots close to a side) near the top.
-    const HostLayout& L = ctx->L;
-    std::vector<std::pair<double, int>> cost;
-    for (int v : L.order) {
-      if (L.knot_boundary[v]) continue;
-      const double* r = L.stencils[L.knot_stencil[v]].rect;
-      const double ax = L.kx[v] - r[0], bx = r[2] - L.kx[v], ay = L.ky[v] - r[1], by = r[3] - L.ky[v];
-      const double tx = 0.5 * std::max(ax * bx, 0.0), ty = 0.5 * std::max(ay * by, 0.0);
-      const double tau = tx + ty > 0.0 ? tx * ty / (tx + ty) : 0.0;
-      const double d = std::min(std::min(ax, bx), std::min(ay, by));
-      double hk = desc->h;
-      if (desc->adaptive_h && d > 1e-4) hk = std::min(hk, std::pow(d / (2.0 * 0.5826 * 1.4142135623730951), 2.0));
-      cost.push_back({-tau / hk, v});
-    }
-    std::stable_sort(cost.begin(), cost.end());
-    std::vector<int> ord;
-    ord.reserve(cost.size());
-    for (auto& c : cost) ord.push_back(c.second);
+    const std::vector<int> ord = geometric_order(ctx, desc, 0, ctx->n_mc);
     CK(ctx->mc_lpt.upload(ord, s));
     ctx->lpt_ready = true;
   }
-  a.mc_knots = (lpt && ctx->lpt_ready) ? ctx->mc_lpt.p : ctx->mc_knots.p + mc0;
+  a.mc_knots = (lpt && ctx->lpt_ready) ? ctx->mc_lpt.p : order ? order : ctx->mc_knots.p + mc0;
   a.item_counter = ctx->counter.p;
   a.Bsum = ctx->Bsum.p;
   a.BBsum = ctx->BBsum.p;
@@ -844,6 +857,17 @@ pdds_status adaptive_continue(pdds_ctx* ctx, const pdds_estimate_desc* desc, con
   return PDDS_OK;
 }
 
+pdds_status order_groups(pdds_ctx* ctx, const pdds_estimate_desc* desc, const std::vector<int>& first) {
+  if (first == ctx->lpt_groups) return PDDS_OK;
+  std::vector<int> all;
+  all.reserve(ctx->n_mc);
+  for (size_t g = 0; g + 1 < first.size(); g++)
+    for (int v : geometric_order(ctx, desc, first[g], first[g + 1] - first[g])) all.push_back(v);
+  CK(ctx->mc_lpt.upload(all, ctx->stream));
+  ctx->lpt_groups = first;
+  return PDDS_OK;
+}
+
 size_t mixed_hist_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int mc_n) {
   int chunks = 1, ppc = 1;
   item_split(ctx, desc->npaths, &chunks, &ppc, tuned_for(ctx, desc) ? ctx->tune_ppc : 0, cta_threads_for(ctx, desc),
@@ -855,7 +879,7 @@ size_t mixed_hist_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int
 }
 
 pdds_status enqueue_mixed(pdds_ctx* ctx, const pdds_estimate_desc* desc, int* launches, int mc0, int mc_n,
-                          bool prefix) {
+                          bool prefix, const int* order) {
   const ProblemDev P = problem_dev(ctx);
   if (prefix) {
     pdds_status st = enqueue_prefix(ctx, desc, P, false, launches);
@@ -866,7 +890,8 @@ pdds_status enqueue_mixed(pdds_ctx* ctx, const pdds_estimate_desc* desc, int* la
   int chunks = 1, ppc = 1;
   item_split(ctx, desc->npaths, &chunks, &ppc, tuned_for(ctx, desc) ? ctx->tune_ppc : 0, cta_threads_for(ctx, desc),
              mc_n);
-  pdds_status st = enqueue_mixed_paths(ctx, desc, P, chunks, ppc, launches, nullptr, mc0, mc_n);
+  pdds_status st = enqueue_mixed_paths(ctx, desc, P, chunks, ppc, launches, nullptr, mc0, mc_n,
+                                       desc->plain_launch ? nullptr : order);
   if (st != PDDS_OK) return st;
   // finalisation of the range's knots: B and BB, and G_var over the range's rows
   const HostLayout& L = ctx->L;

@@ -184,6 +184,7 @@ struct pdds_ctx {
     int i0 = 0, m = 0;
     std::vector<pdds::ResidentPlan> plans;
   } batch_tail;
+  std::vector<int> lpt_groups;  // group bounds (hand-out positions) that mc_lpt is sorted for
   int solve_m = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   // batch of independent instances (pdds_batch_build): the layout above is
@@ -256,9 +257,14 @@ pdds_status check_err_flags(pdds_ctx* ctx);
 // (unless reused), zeroing, boundary knots, the path kernel and the
 // finalisation.  No host synchronisation, so it can be graph-captured.
 // mc0, mc_n: only the knots mc_knots[mc0 .. mc0 + mc_n) (mc_n < 0: to the
-// end); prefix: also the factorisation, zeroing and boundary knots.
+// end); prefix: also the factorisation, zeroing and boundary knots; order:
+// (device) those knots in the order to hand them out.
 pdds_status enqueue_mixed(pdds_ctx* ctx, const pdds_estimate_desc* desc, int* launches, int mc0 = 0,
-                          int mc_n = -1, bool prefix = true);
+                          int mc_n = -1, bool prefix = true, const int* order = nullptr);
+// A batch's hand-out order: the knots at the positions first[g] ..
+// first[g + 1] - 1 (group g), heaviest first, into ctx->mc_lpt at the same
+// positions.  Not while a stream captures.
+pdds_status order_groups(pdds_ctx* ctx, const pdds_estimate_desc* desc, const std::vector<int>& first);
 // Words of exit histograms that enqueue_mixed needs for mc_n knots.
 size_t mixed_hist_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int mc_n);
 // Destroys the captured batch graph (its kernels hold buffer addresses).
