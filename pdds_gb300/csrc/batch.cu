@@ -146,6 +146,8 @@ pdds_status enqueue_batch(pdds_ctx* ctx, const pdds_batch_run_desc* d, int clust
     CK(launch_gmres_cluster(a, cluster, ctx->max_inst_knots, s2));
     ++*launches;
   }
+  st = join_setup(ctx);  // (no knots with paths)
+  if (st != PDDS_OK) return st;
   CK(cudaEventRecord(ctx->wave_ev[W], s2));
   CK(cudaStreamWaitEvent(s, ctx->wave_ev[W], 0));
   return PDDS_OK;
@@ -337,6 +339,10 @@ pdds_status pdds_batch_run(pdds_ctx* ctx, const pdds_batch_run_desc* desc, pdds_
       pdds_status st = enqueue_batch(ctx, desc, cluster, &nl);
       cudaGraph_t g = nullptr;
       cudaError_t ce = cudaStreamEndCapture(s, &g);
+      if (st != PDDS_OK || ce != cudaSuccess) {  // nothing of it ran
+        ctx->setup_pending = false;
+        ctx->tables_ready = false;
+      }
       if (st != PDDS_OK) {
         if (g) cudaGraphDestroy(g);
         return st;

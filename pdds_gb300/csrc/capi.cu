@@ -468,9 +468,20 @@ pdds_status check_err_flags(pdds_ctx* ctx) {
   return PDDS_OK;
 }
 
+pdds_status join_setup(pdds_ctx* ctx) {
+  if (!ctx->setup_pending) return PDDS_OK;
+  ctx->setup_pending = false;
+  CK(cudaStreamWaitEvent(ctx->stream, ctx->setup_ev[1], 0));
+  return PDDS_OK;
+}
+
 pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const ProblemDev& P, bool events,
                            int* launches) {
   cudaStream_t s = ctx->stream;
+  {  // tables of an earlier call that failed before its contraction
+    const pdds_status st = join_setup(ctx);
+    if (st != PDDS_OK) return st;
+  }
   HostLayout& L = ctx->L;
   const int mode = desc->mode;
   const int64_t nnz = L.row_ptr[L.K];
@@ -479,11 +490,30 @@ pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const 
   CK(cudaMemsetAsync(ctx->stats.p, 0, 8 * sizeof(unsigned long long), s));
   const bool need_ipsi = !(mode == PDDS_MODE_REPLAY_FP64 && desc->ipsi_override);
   if (need_ipsi && (!ctx->tables_ready || !desc->reuse_tables)) {
-    int max_n = 0;
-    for (auto& sh : L.shapes) max_n = std::max(max_n, sh.n);
-    CK(launch_rbf_setup(ctx->dl, max_n, ctx->max_nbins, ctx->ipsi.p, ctx->tab.p, ctx->rbf_lu.p, ctx->rbf_piv.p,
-                        ctx->rbf_uinv.p, ctx->errf.p, s));
+    // MIXED paths need no tables: the factorisation (a chain of FP64 steps in
+    // one CTA per shape) runs beside them, at a higher priority so that it is
+    // placed first.  12x12/n43: factorisation 0.38 ms, then 0.25 ms of inverse
+    // and tables in the paths' tail; 741 knots 4.35 -> T741 ms per solve.
+    cudaStream_t sr = s;
+    if (mode == PDDS_MODE_MIXED) {
+      if (!ctx->setup_stream) {
+        int least = 0, greatest = 0;
+        CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        for (cudaEvent_t& ev : ctx->setup_ev)
+          if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        CK(cudaStreamCreateWithPriority(&ctx->setup_stream, cudaStreamNonBlocking, greatest));
+      }
+      sr = ctx->setup_stream;
+      CK(cudaEventRecord(ctx->setup_ev[0], s));
+      CK(cudaStreamWaitEvent(sr, ctx->setup_ev[0], 0));
+    }
+    CK(launch_rbf_setup(ctx->dl, ctx->max_n, ctx->max_nbins, ctx->ipsi.p, ctx->tab.p, ctx->rbf_lu.p, ctx->rbf_piv.p,
+                        ctx->rbf_uinv.p, ctx->errf.p, sr));
     *launches += 4;
+    if (sr != s) {
+      CK(cudaEventRecord(ctx->setup_ev[1], sr));
+      ctx->setup_pending = true;
+    }
     ctx->tables_ready = true;
   }
   if (events) CK(cudaEventRecord(ctx->ev1, s));
@@ -748,6 +778,10 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
       ++*launches;
       ctx->lpt_ready = true;
     }
+    {
+      const pdds_status st = join_setup(ctx);
+      if (st != PDDS_OK) return st;
+    }
     ContractArgs c{};
     c.L = ctx->dl;
     c.hist = ctx->hist.p;
@@ -953,6 +987,7 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->solve_stream) cudaStreamSynchronize(ctx->solve_stream);
+    if (ctx->setup_stream) cudaStreamSynchronize(ctx->setup_stream);
     // both streams are idle: the buffers go to the block cache for the next
     // context
     DBuf<double>* d64[] = {&ctx->kx, &ctx->ky, &ctx->st_rect, &ctx->sd_c, &ctx->sd_origin, &ctx->side_px,
@@ -1021,6 +1056,9 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     ctx->step_hist.recycle();
     for (auto* b : {&ctx->diag, &ctx->rsx, &ctx->rsy, &ctx->rsY, &ctx->rsZ, &ctx->rsxi, &ctx->rknot_h}) b->recycle();
     if (ctx->host_rr) cudaFreeHost(ctx->host_rr);
+    for (cudaEvent_t ev : ctx->setup_ev)
+      if (ev) cudaEventDestroy(ev);
+    if (ctx->setup_stream) cudaStreamDestroy(ctx->setup_stream);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->ev2) cudaEventDestroy(ctx->ev2);
@@ -1480,6 +1518,10 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
                          (mode == PDDS_MODE_MIXED && desc->want_var) ? 1 : 0, s));
     launches += 1 + ((mode == PDDS_MODE_MIXED && desc->want_var) ? 1 : 0);
   }
+  {
+    const pdds_status st = join_setup(ctx);  // (no knots with paths)
+    if (st != PDDS_OK) return st;
+  }
   CK(cudaEventRecord(ctx->ev2, s));
   if (!(mode == PDDS_MODE_MIXED && desc->adaptive_n)) {
     ctx->last_knot_N.assign(L.K, 0);
@@ -1557,6 +1599,7 @@ pdds_status pdds_autotune(pdds_ctx* ctx, const pdds_estimate_desc* desc, int32_t
   d.adaptive_n = 0;
   int launches = 0;
   pdds_status st = enqueue_prefix(ctx, &d, P, false, &launches);
+  if (st == PDDS_OK) st = join_setup(ctx);
   if (st != PDDS_OK) return st;
   // a block size imposed by the caller is kept: only the other shape
   // parameters are searched; 0 searches both block sizes

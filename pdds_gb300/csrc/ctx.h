@@ -187,6 +187,11 @@ struct pdds_ctx {
   std::vector<int> lpt_groups;  // group bounds (hand-out positions) that mc_lpt is sorted for
   int solve_m = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
+  // MIXED: the RBF factorisation and tables run beside the paths, which do
+  // not read them; the contraction waits for setup_ev[1]
+  cudaStream_t setup_stream = nullptr;
+  cudaEvent_t setup_ev[2] = {nullptr, nullptr};
+  bool setup_pending = false;
   // batch of independent instances (pdds_batch_build): the layout above is
   // the block-diagonal union of the instances' layouts
   bool is_batch = false;
@@ -265,6 +270,8 @@ pdds_status enqueue_mixed(pdds_ctx* ctx, const pdds_estimate_desc* desc, int* la
 // first[g + 1] - 1 (group g), heaviest first, into ctx->mc_lpt at the same
 // positions.  Not while a stream captures.
 pdds_status order_groups(pdds_ctx* ctx, const pdds_estimate_desc* desc, const std::vector<int>& first);
+// Makes ctx->stream wait for the tables of this call's prefix.
+pdds_status join_setup(pdds_ctx* ctx);
 // Words of exit histograms that enqueue_mixed needs for mc_n knots.
 size_t mixed_hist_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int mc_n);
 // Destroys the captured batch graph (its kernels hold buffer addresses).
