@@ -493,8 +493,11 @@ pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const 
     // one CTA per shape) runs beside them, at a higher priority so that it is
     // placed first.  12x12/n43: factorisation 0.38 ms, then 0.25 ms of inverse
     // and tables in the paths' tail; 741 knots 4.35 -> 4.03 ms per solve, 237 knots 782 -> 717 us.
+    // Not beside table-served paths, which live on the L1: the SMs that ran the
+    // factorisation (up to 127 KB of shared memory) keep a small one for the
+    // whole launch (8x8/n31, 1024^2 table, 207.5 -> 214 ms).
     cudaStream_t sr = s;
-    if (mode == PDDS_MODE_MIXED) {
+    if (mode == PDDS_MODE_MIXED && P.kind != PK_LUT) {
       if (!ctx->setup_stream) {
         int least = 0, greatest = 0;
         CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
