@@ -986,7 +986,7 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     DBuf<double>* d64[] = {&ctx->kx, &ctx->ky, &ctx->st_rect, &ctx->sd_c, &ctx->sd_origin, &ctx->side_px,
                            &ctx->side_py, &ctx->sh_c, &ctx->sh_R, &ctx->sh_lo, &ctx->sh_delta, &ctx->sh_t, &ctx->ipsi,
                            &ctx->G, &ctx->GG, &ctx->B, &ctx->BB, &ctx->Bsum, &ctx->BBsum, &ctx->rx,
-                           &ctx->ry, &ctx->rY, &ctx->rZ, &ctx->rxi, &ctx->Gside, &ctx->GGside,
+                           &ctx->ry, &ctx->rY, &ctx->rZ, &ctx->rxi, &ctx->Gside, &ctx->GGside, &ctx->rhy,
                            &ctx->ipsi_knot, &ctx->sv64, &ctx->sscal, &ctx->spart, &ctx->shess, &ctx->su,
                            &ctx->rbf_lu, &ctx->rbf_uinv};
     for (auto* b : d64) b->recycle();
@@ -1434,8 +1434,10 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
     a.dup_sum = ctx->L.geom == 1 ? 1 : desc->dup_sum;  // circle layouts sum shared side knots
     a.err_flags = ctx->errf.p;
     CK(launch_replay_paths(a, P.kind, ctx->num_sms, s));
-    CK(launch_replay_reduce(a, P.kind, max_n, ctx->knot_task_off.p, ctx->Gside.p, ctx->GGside.p, s));
-    launches += 5;
+    CK(ctx->rhy.resize(std::max<size_t>(1, (size_t)rn * replay_terms_paths(rn, N, max_n) * max_n)));
+    CK(launch_replay_reduce(a, P.kind, max_n, ctx->knot_task_off.p, ctx->Gside.p, ctx->GGside.p, ctx->rhy.p,
+                            &launches, s));
+    launches += 4;
   } else {
     int chunks = 1, ppc = 1;
     item_split(ctx, N, &chunks, &ppc, (mode == PDDS_MODE_MIXED && tuned_for(ctx, desc)) ? ctx->tune_ppc : 0,

@@ -160,7 +160,7 @@ struct pdds_ctx {
   DBuf<int> counter;
   bool has_estimate = false;
   // replay scratch
-  DBuf<double> rx, ry, rY, rZ, rxi, Gside, GGside, ipsi_knot;
+  DBuf<double> rx, ry, rY, rZ, rxi, Gside, GGside, rhy, ipsi_knot;
   DBuf<int> rside, rsl, rss;
   DBuf<int64_t> knot_task_off, knot_ipsi_off;
   // solve scratch

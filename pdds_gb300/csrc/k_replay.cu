@@ -431,21 +431,93 @@ __global__ void __launch_bounds__(RB_CHUNK) k_replay_b(const ReplayArgs a) {
   }
 }
 
-// G_update accumulation for one (knot, side), paths in order: the side's
-// exits are collected in path order, RG_EXITS at a time; the CTA forms their
-// RBF values r_j (each used by every side knot; the per-knot loop this
-// replaces took the n exponentials anew for each of the n knots), then
-// H_i Y = (sum_j ipsi(j, i) r_j) Y with j in order, and one thread per side
-// knot adds the exits' terms in order.
+// G_update accumulation in two launches, for paths [p0, p1) of every knot.
+//
+// First the exits' terms H_i Y, in any order: a CTA collects the exits of one
+// (knot, side, RG_PATHS paths), RG_EXITS at a time, forms their RBF values r_j
+// (each used by every side knot; the per-knot loop this replaces took the n
+// exponentials anew for each of the n knots), then
+// H_i Y = (sum_j ipsi(j, i) r_j) Y with j in order, into hy[path][i].  FP64
+// instructions bound it, so it has to fill every SM: with a CTA per (knot,
+// side) and all of its paths, which also added the terms, the side nearest to
+// its knot (nine tenths of the exits) set the end: 26.3 ms at 225 knots x 10^4
+// paths; the two launches take 10.5 and 1.6 ms.
 constexpr int RG_THREADS = 256;
 constexpr int RG_EXITS = 32;
+constexpr int RG_PATHS = 512;
 
-__global__ void __launch_bounds__(RG_THREADS) k_replay_g(const ReplayArgs a, const int64_t* knot_task_off,
-                                                        double* Gside, double* GGside) {
-  extern __shared__ double dyn[];  // r [RG_EXITS][n], then H Y [RG_EXITS][n]
-  __shared__ int queue[RG_EXITS + RG_THREADS];
+__global__ void __launch_bounds__(RG_THREADS) k_replay_terms(const ReplayArgs a, int p0, int p1, double* hy, int ld) {
+  extern __shared__ double r[];  // [RG_EXITS][n]
+  __shared__ int queue[RG_PATHS];
   __shared__ int s_cnt[RG_THREADS / 32];
   __shared__ double s_x[RG_EXITS], s_y[RG_EXITS], s_Y[RG_EXITS];
+  const int m = blockIdx.x, d = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const DevLayout& L = a.L;
+  const int sd = L.st_side[4 * L.knot_stencil[a.mc_knots[m]] + d];
+  if (sd < 0) return;
+  const int n = L.sd_n[sd];
+  const double c = L.sd_c[sd];
+  const double c2 = c * c;
+  const double* px = L.side_px + L.sd_knot_off[sd];
+  const double* py = L.side_py + L.sd_knot_off[sd];
+  const double* ip = a.knot_ipsi_off ? a.ipsi_knot + a.knot_ipsi_off[4 * m + d]
+                                     : L.ipsi + L.sh_ipsi_off[L.sd_shape[sd]];
+  const int b0 = p0 + blockIdx.z * RG_PATHS, b1 = min(p1, b0 + RG_PATHS);
+  int all = 0;
+  for (int q0 = b0; q0 < b1; q0 += RG_THREADS) {
+    const int p = q0 + tid;
+    const bool hit = p < b1 && a.eside[(int64_t)m * a.N + p] == d;
+    const unsigned mk = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) s_cnt[warp] = __popc(mk);
+    __syncthreads();
+    int at = all + __popc(mk & ((1u << lane) - 1u));
+    for (int w = 0; w < RG_THREADS / 32; w++) {
+      if (w < warp) at += s_cnt[w];
+      all += s_cnt[w];
+    }
+    if (hit) queue[at] = p;
+    __syncthreads();
+  }
+  for (int q0 = 0; q0 < all; q0 += RG_EXITS) {
+    const int ne = min(RG_EXITS, all - q0);
+    if (tid < ne) {
+      const int64_t o = (int64_t)m * a.N + queue[q0 + tid];
+      s_x[tid] = a.ex[o];
+      s_y[tid] = a.ey[o];
+      s_Y[tid] = a.eY[o];
+    }
+    __syncthreads();
+    for (int e = tid; e < ne * n; e += RG_THREADS) {
+      const int x = e / n, j = e - x * n;
+      // the RBF of the reference (BVPs/BVP.hpp:84-87), c^2 formed once
+      const double d0 = px[j] - s_x[x], d1 = py[j] - s_y[x];
+      const double nrm = ::sqrt(d0 * d0 + d1 * d1);
+      r[e] = pm::exp(-(nrm * nrm) / c2);
+    }
+    __syncthreads();
+    for (int e = tid; e < ne * n; e += RG_THREADS) {
+      const int x = e / n, i = e - x * n;
+      const double* rx = r + x * n;
+      double H = 0.0;
+#pragma unroll 4
+      for (int j = 0; j < n; j++) H += __ldg(ip + (int64_t)j * n + i) * rx[j];
+      hy[((int64_t)m * (p1 - p0) + queue[q0 + x] - p0) * ld + i] = H * s_Y[x];
+    }
+    __syncthreads();
+  }
+}
+
+// Then their sums in path order, a thread per (knot, side, side knot): a
+// chain of additions, fed by loads RS_AHEAD exits ahead.
+constexpr int RS_THREADS = 160;  // side knots of a stencil side, at most
+constexpr int RS_PATHS = 640;
+constexpr int RS_AHEAD = 16;
+
+__global__ void __launch_bounds__(RS_THREADS) k_replay_sum(const ReplayArgs a, int p0, int p1, const double* hy, int ld,
+                                                          const int64_t* knot_task_off, double* Gside,
+                                                          double* GGside) {
+  __shared__ int queue[RS_PATHS];
+  __shared__ int s_cnt[RS_THREADS / 32];
   const int m = blockIdx.x, d = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const DevLayout& L = a.L;
   const int st = L.knot_stencil[a.mc_knots[m]];
@@ -457,74 +529,50 @@ __global__ void __launch_bounds__(RG_THREADS) k_replay_g(const ReplayArgs a, con
     if (s2 >= 0) out += L.sd_n[s2];
   }
   const int n = L.sd_n[sd];
-  const double c = L.sd_c[sd];
-  const double c2 = c * c;
-  const double* px = L.side_px + L.sd_knot_off[sd];
-  const double* py = L.side_py + L.sd_knot_off[sd];
-  const double* ip = a.knot_ipsi_off ? a.ipsi_knot + a.knot_ipsi_off[4 * m + d]
-                                     : L.ipsi + L.sh_ipsi_off[L.sd_shape[sd]];
-  double* r = dyn;
-  double* hy = dyn + RG_EXITS * n;
+  const bool mine = tid < n;
   double G = 0.0, GG = 0.0;  // of side knot tid
-  int nq = 0;                // queued exits
-  for (int p0 = 0; p0 < a.N; p0 += RG_THREADS) {
-    const int p = p0 + tid;
-    const bool hit = p < a.N && a.eside[(int64_t)m * a.N + p] == d;
-    const unsigned mk = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) s_cnt[warp] = __popc(mk);
-    __syncthreads();
-    int at = nq + __popc(mk & ((1u << lane) - 1u)), all = nq;
-    for (int w = 0; w < RG_THREADS / 32; w++) {
-      if (w < warp) at += s_cnt[w];
-      all += s_cnt[w];
-    }
-    if (hit) queue[at] = p;
-    __syncthreads();
-    const bool last = p0 + RG_THREADS >= a.N;
-    int q0 = 0;
-    while (all - q0 >= RG_EXITS || (last && all > q0)) {
-      const int ne = min(RG_EXITS, all - q0);
-      if (tid < ne) {
-        const int64_t o = (int64_t)m * a.N + queue[q0 + tid];
-        s_x[tid] = a.ex[o];
-        s_y[tid] = a.ey[o];
-        s_Y[tid] = a.eY[o];
-      }
-      __syncthreads();
-      for (int e = tid; e < ne * n; e += RG_THREADS) {
-        const int x = e / n, j = e - x * n;
-        // the RBF of the reference (BVPs/BVP.hpp:84-87), c^2 formed once
-        const double d0 = px[j] - s_x[x], d1 = py[j] - s_y[x];
-        const double nrm = ::sqrt(d0 * d0 + d1 * d1);
-        r[e] = pm::exp(-(nrm * nrm) / c2);
-      }
-      __syncthreads();
-      for (int e = tid; e < ne * n; e += RG_THREADS) {
-        const int x = e / n, i = e - x * n;
-        const double* rx = r + x * n;
-        double H = 0.0;
-#pragma unroll 4
-        for (int j = 0; j < n; j++) H += __ldg(ip + (int64_t)j * n + i) * rx[j];
-        hy[e] = H * s_Y[x];
-      }
-      __syncthreads();
-      if (tid < n)
-        for (int x = 0; x < ne; x++) {
-          const double t = hy[x * n + tid];
-          G -= t;
-          GG += t * t;
-        }
-      q0 += ne;
-    }
-    // exits left over move to the front
-    const int left = all - q0;
-    int keep = 0;
-    if (tid < left) keep = queue[q0 + tid];
-    __syncthreads();
-    if (tid < left) queue[tid] = keep;
-    nq = left;
+  if (mine && p0 > 0) {
+    G = Gside[out + tid];
+    GG = GGside[out + tid];
   }
-  if (tid < n) {
+  const double* h0 = hy + (int64_t)m * (p1 - p0) * ld + tid;
+  for (int b0 = p0; b0 < p1; b0 += RS_PATHS) {
+    int all = 0;
+    for (int q0 = b0; q0 < min(p1, b0 + RS_PATHS); q0 += RS_THREADS) {
+      const int p = q0 + tid;
+      const bool hit = p < p1 && a.eside[(int64_t)m * a.N + p] == d;
+      const unsigned mk = __ballot_sync(0xffffffffu, hit);
+      if (lane == 0) s_cnt[warp] = __popc(mk);
+      __syncthreads();
+      int at = all + __popc(mk & ((1u << lane) - 1u));
+      for (int w = 0; w < RS_THREADS / 32; w++) {
+        if (w < warp) at += s_cnt[w];
+        all += s_cnt[w];
+      }
+      if (hit) queue[at] = p - p0;
+      __syncthreads();
+    }
+    if (mine) {
+      double t[RS_AHEAD];
+      int q = 0;
+      for (; q + RS_AHEAD <= all; q += RS_AHEAD) {
+#pragma unroll
+        for (int u = 0; u < RS_AHEAD; u++) t[u] = __ldcs(h0 + (int64_t)queue[q + u] * ld);
+#pragma unroll
+        for (int u = 0; u < RS_AHEAD; u++) {
+          G -= t[u];
+          GG += t[u] * t[u];
+        }
+      }
+      for (; q < all; q++) {
+        const double v = __ldcs(h0 + (int64_t)queue[q] * ld);
+        G -= v;
+        GG += v * v;
+      }
+    }
+    __syncthreads();
+  }
+  if (mine) {
     Gside[out + tid] = G;
     GGside[out + tid] = GG;
   }
@@ -594,8 +642,16 @@ static void launch_b_t(const ReplayArgs& a, cudaStream_t s) {
   k_replay_b<KIND><<<a.n_mc, RB_CHUNK, smem, s>>>(a);
 }
 
+int replay_terms_paths(int n_mc, int N, int max_n) {
+  // 512 MB of terms, but at least 128 paths, and at most 65,535 blocks of
+  // paths (the grid's z)
+  const int64_t per_path = std::max<int64_t>(1, (int64_t)n_mc * max_n * (int64_t)sizeof(double));
+  const int64_t fit = std::max<int64_t>(128, ((int64_t)512 << 20) / per_path);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(N, (int64_t)65535 * RG_PATHS), fit));
+}
+
 cudaError_t launch_replay_reduce(const ReplayArgs& a, int kind, int max_n, const int64_t* knot_task_off,
-                                 double* Gside, double* GGside, cudaStream_t s) {
+                                 double* Gside, double* GGside, double* hy, int* launches, cudaStream_t s) {
   if (a.n_mc == 0) return cudaSuccess;
   switch (kind) {
     case PK_POISSON_SINCOS: launch_b_t<PK_POISSON_SINCOS>(a, s); break;
@@ -604,11 +660,19 @@ cudaError_t launch_replay_reduce(const ReplayArgs& a, int kind, int max_n, const
     case PK_LUT: launch_b_t<PK_LUT>(a, s); break;
     default: return cudaErrorInvalidValue;
   }
+  if (max_n > RS_THREADS) return cudaErrorInvalidValue;
   if (max_n > 0) {
-    const size_t smem = (size_t)2 * RG_EXITS * max_n * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(k_replay_g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = (size_t)RG_EXITS * max_n * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(k_replay_terms, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_replay_g<<<dim3(a.n_mc, 4), RG_THREADS, smem, s>>>(a, knot_task_off, Gside, GGside);
+    const int part = replay_terms_paths(a.n_mc, a.N, max_n);
+    for (int p0 = 0; p0 < a.N; p0 += part) {
+      const int p1 = std::min(a.N, p0 + part);
+      const int blocks = (p1 - p0 + RG_PATHS - 1) / RG_PATHS;
+      k_replay_terms<<<dim3(a.n_mc, 4, blocks), RG_THREADS, smem, s>>>(a, p0, p1, hy, max_n);
+      k_replay_sum<<<dim3(a.n_mc, 4), RS_THREADS, 0, s>>>(a, p0, p1, hy, max_n, knot_task_off, Gside, GGside);
+      *launches += 2;
+    }
   }
   k_replay_row<<<(a.n_mc + 127) / 128, 128, 0, s>>>(a, knot_task_off, Gside, GGside);
   return cudaGetLastError();

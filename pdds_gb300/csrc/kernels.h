@@ -233,7 +233,9 @@ cudaError_t launch_replay_paths(const ReplayArgs& a, int kind, int num_sms, cuda
 // max_n: side knots of the largest side; knot_task_off: first side entry of
 // each knot in Gside and GGside (sides N, S, E, W one after the other)
 cudaError_t launch_replay_reduce(const ReplayArgs& a, int kind, int max_n, const int64_t* knot_task_off,
-                                 double* Gside, double* GGside, cudaStream_t s);
+                                 double* Gside, double* GGside, double* hy, int* launches, cudaStream_t s);
+// paths whose RBF terms are held at once: hy has n_mc x that x max_n words
+int replay_terms_paths(int n_mc, int N, int max_n);
 // FP64 factorisation of every shape's Psi and the cardinal-function tables.
 // lu: scratch of the ipsi layout; piv, uinv: scratch of the sh_t layout
 cudaError_t launch_rbf_setup(const DevLayout& L, int max_n, int max_nbins, double* ipsi, float* tab,
