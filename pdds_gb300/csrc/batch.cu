@@ -30,12 +30,13 @@ int batch_waves(const pdds_ctx* ctx, const pdds_batch_run_desc* d) {
 // system on chip (k_resident.cu), which takes all SMs: nothing else is left
 // to run beside that group's solves, while the cluster kernel (16 SMs per
 // system) leaves most of the chip idle.  A batch of 24 whose last group has
-// 14,952 and 19,005 rows ends 9.6 ms earlier (147.9 -> 138.4 ms).  Not for
-// many systems at once, which fill the chip: one system takes a third (237
-// rows) to a seventh (19,005 rows) of the cluster kernel's time, but one
-// follows the other, and the cluster kernel runs num_sms / cluster at a time.
-// The classical form and systems that do not fit keep the cluster.
-constexpr int TAIL_GAIN = 3;
+// 14,952 and 19,005 rows ends 9.6 ms earlier (147.9 -> 138.4 ms), with three
+// in it (10 groups) 10 ms.  Not for many systems at once, which fill the
+// chip: one takes a third (237 rows) to a ninth (19,005 rows) of the cluster
+// kernel's time, but one follows the other, and the cluster kernel runs
+// num_sms / cluster at a time.  The classical form and systems that do not
+// fit keep the cluster.
+int tail_systems(int max_rows) { return 3 + max_rows / 3000; }
 const std::vector<ResidentPlan>& batch_tail(pdds_ctx* ctx, const pdds_batch_run_desc* d, int cluster, int i0, int m) {
   pdds_ctx::BatchTail& t = ctx->batch_tail;
   if (!t.ready || t.i0 != i0 || t.m != m) {
@@ -45,7 +46,10 @@ const std::vector<ResidentPlan>& batch_tail(pdds_ctx* ctx, const pdds_batch_run_
     t.ready = true;
     const int n = ctx->n_inst - i0;
     const int rounds = (n * cluster + ctx->num_sms - 1) / std::max(ctx->num_sms, 1);
-    for (int i = i0; i < ctx->n_inst && n <= TAIL_GAIN * rounds; i++) {
+    int rows_max = 0;
+    for (int i = i0; i < ctx->n_inst; i++) rows_max = std::max(rows_max, ctx->inst_k0[i + 1] - ctx->inst_k0[i]);
+    const int64_t most = (int64_t)rounds * tail_systems(rows_max);
+    for (int i = i0; i < ctx->n_inst && n <= most; i++) {
       const int k0 = ctx->inst_k0[i];
       const ResidentRows rows{ctx->inst_k0[i + 1] - k0, ctx->L.row_ptr.data() + k0, ctx->L.knot_stencil.data() + k0};
       t.plans.push_back(resident_plan(rows, RESIDENT_GMRES, m, 0));
