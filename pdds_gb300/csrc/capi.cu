@@ -650,6 +650,26 @@ std::vector<int> geometric_order(const pdds_ctx* ctx, const pdds_estimate_desc* 
   return ord;
 }
 
+// Whether 256-thread CTAs, the default below 8,192 knots, are better halved
+// for items of ppc paths: at an item's end a CTA waits for the longest of its
+// lanes' paths, so short items (a few paths per lane) want fewer lanes each,
+// and 2.25 items or more per 128-thread CTA, so that the launch's end does
+// not weigh more.  Path kernel with 128 threads against 256, 112 to 2,177
+// knots, three problems, the same items: up to 1,250 paths per item 0.68 to
+// 1.0 (mean 0.87), from 1,666 on 0.83 to 1.2.  Richardson pairs lose (1.05 to
+// 1.1) where their queues and histograms leave fewer lanes per SM.  Table
+// kinds and polar stencils were not measured and stay.
+bool short_items(const pdds_ctx* ctx, const MixedArgs& a, int mk, int n_items, int ppc, int threads) {
+  if (threads != 256 || ctx->L.geom != 0 || mk == PK_LUT || mk == PK_LUT_TEX) return false;
+  if (ppc > 1300 || 4 * (int64_t)n_items < 9 * 8 * (int64_t)ctx->num_sms) return false;
+  if (!a.richardson) return true;
+  auto lanes = [&](int th) {
+    const size_t smem = ctx->mixed_smem * (a.want_var ? 2 : 1) + mixed_queue_smem(th, a.richardson);
+    return th * mixed_blocks_per_sm(mk, smem, a.richardson, th, a.diag != nullptr);
+  };
+  return lanes(128) >= lanes(256);
+}
+
 pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, const ProblemDev& P, int chunks,
                                 int ppc, int* launches, const ItemList* items = nullptr, int mc0 = 0,
                                 int mc_n = -1, const int* order = nullptr) {
@@ -751,7 +771,11 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   a.knot_steps = ctx->knot_steps.p;
   a.step_hist = desc->step_histogram ? ctx->step_hist.p : nullptr;
   a.diag = (desc->diagnostics && ctx->diag.n >= (size_t)ctx->L.K * PDDS_DIAG_N) ? ctx->diag.p : nullptr;
-  const int threads = cta_threads_for(ctx, desc);
+  const int mk = mixed_kind(P);
+  int threads = cta_threads_for(ctx, desc);
+  if (!items && desc->cta_threads == 0 && !tuned_for(ctx, desc) && short_items(ctx, a, mk, n_items, ppc, threads))
+    threads = 128;
+  if (!items) ctx->run_threads = threads;
   const size_t base_smem = ctx->mixed_smem * (a.want_var ? 2 : 1) + mixed_queue_smem(threads, a.richardson);
   a.hist_cap = (int)(ctx->mixed_smem / sizeof(float));
   a.hist_stride = slot_words(ctx, desc);
@@ -760,7 +784,6 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   a.hist_out = ctx->hist.p;
   a.mc_pos = ctx->mc_pos.p;
   a.mc0 = mc0;
-  const int mk = mixed_kind(P);
   const size_t smem = base_smem + (mk == PK_LUT ? lut_stage(ctx, P, base_smem, threads, &a.lut_nodes) : 0);
   if (smem > 200 * 1024) return fail(ctx, PDDS_ERR_INVALID, "exit histograms exceed shared memory; lower bins_per_gap");
   int bps = mixed_blocks_per_sm(mk, smem, a.richardson, threads, a.diag != nullptr);
@@ -1553,7 +1576,7 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
     info->path_steps = (int64_t)st[0];
     info->exits_global = (int64_t)st[2];
     info->exits_stencil = (int64_t)st[3];
-    info->cta_threads = mode == PDDS_MODE_MIXED ? cta_threads_for(ctx, desc) : 0;
+    info->cta_threads = mode == PDDS_MODE_MIXED ? ctx->run_threads : 0;
   }
   const pdds_status fst = check_err_flags(ctx);
   if (info) {

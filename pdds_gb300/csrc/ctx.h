@@ -147,6 +147,7 @@ struct pdds_ctx {
   int n_mc = 0, n_bnd = 0;
   std::vector<int> mc_host;  // knots with paths, in hand-out order (the device mc_knots)
   size_t mixed_smem = 0;
+  int run_threads = 0;            // CTA size of the last MIXED estimate's path kernel
   int fp64_nall = 0;              // side knots of the largest stencil
   int max_n = 0, max_nbins = 0;   // of the shapes
   // exit histograms of a MIXED launch's work items, and an item list's knots
