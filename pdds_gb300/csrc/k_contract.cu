@@ -278,6 +278,9 @@ __global__ void __launch_bounds__(Tile<VAR>::THREADS, VAR ? 2 : 3) k_contract(co
 
 }  // namespace
 
+// three stages of 32 bins x 160 columns and both histograms, with room
+constexpr int CT_SMEM_MAX = 96 * 1024;
+
 cudaError_t launch_contract(const ContractArgs& a, int max_n, int max_nbins, int num_sms, int* launches,
                             cudaStream_t s) {
   if (a.n_rows < 1 || max_n < 1) return cudaSuccess;
@@ -289,7 +292,8 @@ cudaError_t launch_contract(const ContractArgs& a, int max_n, int max_nbins, int
   auto run = [&](auto kernel, int threads, int a_words) -> cudaError_t {
     const int stage_words = a_words + ((CT_BINS * max_n + 3) & ~3);
     const size_t smem = ((size_t)CT_RING * stage_words + 128) * sizeof(float);
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > CT_SMEM_MAX) return cudaErrorInvalidValue;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM_MAX);
     if (e != cudaSuccess) return e;
     kernel<<<grid, threads, smem, s>>>(a, stage_words);
     ++*launches;

@@ -931,11 +931,16 @@ k_paths_mixed(const MixedArgs a) {
 
 }  // namespace
 
+// Dynamic shared memory that any launch may ask for (enqueue_mixed_paths
+// refuses more).  The kernels' limit is always set to this: a smaller one, set
+// for another launch, would refuse a captured node's new parameters.
+constexpr int MIXED_SMEM_MAX = 200 * 1024;
+
 // Polar stencils are instantiated for the isotropic problems only.
 template <bool RICH>
 static cudaError_t launch_mixed_t(const MixedArgs& a, int kind, int grid, int threads, size_t smem, cudaStream_t s) {
 #define PDDS_MIXED_LAUNCH(KK, GG, DD)                                                                         \
-  cudaFuncSetAttribute(k_paths_mixed<KK, RICH, GG, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+  cudaFuncSetAttribute(k_paths_mixed<KK, RICH, GG, DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, MIXED_SMEM_MAX); \
   k_paths_mixed<KK, RICH, GG, DD><<<grid, threads, smem, s>>>(a);
 #define PDDS_MIXED_CASE(KK, GG)            \
   case KK:                                 \
@@ -1025,7 +1030,7 @@ static int blocks_t(int kind, size_t smem, int threads) {
   int nb = 0;
 #define PDDS_OCC(KK)                                                                                          \
   case KK:                                                                                                    \
-    cudaFuncSetAttribute(k_paths_mixed<KK, RICH, 0, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    cudaFuncSetAttribute(k_paths_mixed<KK, RICH, 0, DIAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, MIXED_SMEM_MAX); \
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_paths_mixed<KK, RICH, 0, DIAG>, threads, smem);       \
     break;
   switch (kind) {

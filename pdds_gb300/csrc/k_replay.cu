@@ -662,9 +662,7 @@ cudaError_t launch_replay_reduce(const ReplayArgs& a, int kind, int max_n, const
   }
   if (max_n > RS_THREADS) return cudaErrorInvalidValue;
   if (max_n > 0) {
-    const size_t smem = (size_t)RG_EXITS * max_n * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(k_replay_terms, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    const size_t smem = (size_t)RG_EXITS * max_n * sizeof(double);  // at most 40 KB
     const int part = replay_terms_paths(a.n_mc, a.N, max_n);
     for (int p0 = 0; p0 < a.N; p0 += part) {
       const int p1 = std::min(a.N, p0 + part);

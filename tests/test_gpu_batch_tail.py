@@ -36,3 +36,18 @@ def test_entries_beyond_the_chip():
         assert info["kernel_launches"] == 1 and info["rel_residual"] <= 1e-10
         # a relative residual of 1e-10, amplified by less than the rows' count over the diagonal's dominance
         assert np.max(np.abs(u - v)) <= 1e-6 * np.max(np.abs(v))
+
+
+def test_graph_replay_after_other_launch_shapes():
+    """Path kernels of different CTA sizes and shared memory, launched in between, do not spoil a captured batch."""
+    insts = batch_instances(2, seed=5, grid=(5, 6), nodes=(12, 15))
+    opts = dict(richardson=True, dup_sum=True, use_graph=True)
+    with P.Batch(P.BVP.HELMHOLTZ, insts) as b, P.PDDSparseGM((0.0, 0.0), (1.0, 1.0), 3, 5, fac_rule(1.0, 3, 5)) as pd:
+        b.run(5000, 2e-3, seed=3, **opts)
+        u = b.result(1)["u"].copy()
+        for th in (128, 256):
+            pd.estimate(P.BVP.helmholtz(2.0, 1.0, -1.0), 300, 2e-3, cta_threads=th, richardson=True)
+        info = b.run(5000, 2e-3, seed=3, **opts)
+        assert info["graph_replayed"] == 1
+        # the order of FP32 sums, as in the tests above
+        assert np.max(np.abs(b.result(1)["u"] - u)) <= 1e-5 * np.max(np.abs(u))
