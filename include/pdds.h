@@ -287,7 +287,9 @@ typedef struct {
   int64_t paths;         /* simulated paths                              */
   int64_t exits_global;  /* exits on the domain boundary                 */
   int64_t exits_stencil; /* exits on interior stencil sides              */
-  double ms_setup;       /* factorisation and tables                     */
+  double ms_setup;       /* before the paths: factorisation and tables,
+                            which MIXED mode runs beside the paths (except
+                            for table-served problems)                   */
   double ms_paths;       /* path kernels and reduction                   */
   int32_t kernel_launches;
   int32_t cta_threads;   /* MIXED: threads per CTA of the path kernel    */
@@ -484,7 +486,8 @@ typedef struct {
   /* the instances run in this many consecutive groups of the order given to
    * pdds_batch_build (0 = 16, at most the instance count): one path-kernel
    * launch per group, and the solves of a group, on a second stream of
-   * higher priority, overlap the next group's paths, so an instance
+   * higher priority, overlap the next group's paths (a few systems of the
+   * last group run one after another on the whole GPU), so an instance
    * completes when its group does; instances given smallest first complete
    * soonest on average */
   int32_t waves;

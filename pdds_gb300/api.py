@@ -825,7 +825,8 @@ class Batch:
     No counterpart in the reference, whose PDDSparseGM solves one problem per
     run.  The instances run in waves (consecutive groups in processing
     order): one path-kernel launch per wave, and one cluster-GMRES launch per
-    wave on a higher-priority stream while the next wave's paths run; with
+    wave on a higher-priority stream while the next wave's paths run (a few
+    systems of the last wave run one after another on the whole GPU); with
     use_graph=True the sequence is captured once in a CUDA graph and
     replayed.  order="smallest_first" processes the instances by increasing
     knot count, so the small ones finish in the first waves (lower median

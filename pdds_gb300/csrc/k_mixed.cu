@@ -10,8 +10,8 @@
 // at full width and needs no bookkeeping across lanes.  An exit
 // on an interior stencil side deposits Y with cubic Lagrange weights into a
 // per-side histogram of the exit coordinate in shared memory (4 FP32 atomics,
-// O(1) per exit).  At the end of
-// the item the histograms are contracted with the FP32 table of cardinal
+// O(1) per exit).  At the end of the item the histograms are written out, and
+// k_contract (k_contract.cu) contracts them with the FP32 table of cardinal
 // functions H_i(s) = sum_j Psi^-1(j,i) exp(-(t_j - s)^2 / c^2), computed in
 // FP64 from the factorised RBF matrix, and added into the G row in FP64.
 // This is the same estimator as the reference's per-exit G_update

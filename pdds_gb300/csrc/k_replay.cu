@@ -22,7 +22,7 @@
 // threshold is not.
 //
 // 4x4/n11, N = 1e4, h = 1e-3 (one thread per path, and one per side knot that
-// walked every path, -> now): paths 216 -> 38 ms, G 626 -> 26 ms, B 43 -> 1.0 ms.
+// walked every path, -> now): paths 216 -> 38 ms, G 626 -> 12 ms, B 43 -> 1.0 ms.
 #include <algorithm>
 
 #include "dev_common.cuh"
