@@ -485,8 +485,18 @@ pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const 
   const int mode = desc->mode;
   const int64_t nnz = L.row_ptr[L.K];
   if (events) CK(cudaEventRecord(ctx->ev0, s));
-  CK(cudaMemsetAsync(ctx->errf.p, 0, sizeof(unsigned), s));
-  CK(cudaMemsetAsync(ctx->stats.p, 0, 8 * sizeof(unsigned long long), s));
+  CK(ctx->step_hist.resize(32));
+  ZeroList z;
+  z.add(ctx->errf.p, 1);
+  z.add(ctx->stats.p, 8);
+  z.add(ctx->G.p, std::max<int64_t>(nnz, 1));
+  z.add(ctx->GG.p, std::max<int64_t>(nnz, 1));
+  z.add(ctx->Bsum.p, L.K);
+  z.add(ctx->BBsum.p, L.K);
+  z.add(ctx->knot_steps.p, L.K);
+  z.add(ctx->step_hist.p, 32);
+  CK(launch_zero(z, ctx->num_sms, s));
+  ++*launches;
   const bool need_ipsi = !(mode == PDDS_MODE_REPLAY_FP64 && desc->ipsi_override);
   if (need_ipsi && (!ctx->tables_ready || !desc->reuse_tables)) {
     // MIXED paths need no tables: the factorisation (a chain of FP64 steps in
@@ -519,13 +529,6 @@ pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const 
     ctx->tables_ready = true;
   }
   if (events) CK(cudaEventRecord(ctx->ev1, s));
-  CK(cudaMemsetAsync(ctx->G.p, 0, std::max<int64_t>(nnz, 1) * sizeof(double), s));
-  CK(cudaMemsetAsync(ctx->GG.p, 0, std::max<int64_t>(nnz, 1) * sizeof(double), s));
-  CK(cudaMemsetAsync(ctx->Bsum.p, 0, L.K * sizeof(double), s));
-  CK(cudaMemsetAsync(ctx->BBsum.p, 0, L.K * sizeof(double), s));
-  CK(cudaMemsetAsync(ctx->knot_steps.p, 0, L.K * sizeof(unsigned long long), s));
-  CK(ctx->step_hist.resize(32));
-  CK(cudaMemsetAsync(ctx->step_hist.p, 0, 32 * sizeof(unsigned long long), s));
   ctx->has_knot_steps = (mode == PDDS_MODE_MIXED);
   CK(launch_boundary_b(ctx->dl, P, mode, ctx->bnd_knots.p, ctx->n_bnd, ctx->B.p, ctx->BB.p, s));
   *launches += ctx->n_bnd > 0;
@@ -1369,6 +1372,7 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
   const ProblemDev P = problem_dev(ctx);
   const int N = desc->npaths;
   int launches = 0;
+  ctx->run_threads = cta_threads_for(ctx, desc);
   {
     pdds_status st = enqueue_prefix(ctx, desc, P, true, &launches);
     if (st != PDDS_OK) return st;

@@ -210,6 +210,20 @@ size_t mixed_queue_smem(int threads, int richardson);
 // max_n, max_nbins: of the layout's shapes
 cudaError_t launch_contract(const ContractArgs& a, int max_n, int max_nbins, int num_sms, int* launches,
                             cudaStream_t s);
+// Buffers to be zeroed in one launch (4-byte words each, 4-byte aligned).
+struct ZeroList {
+  static constexpr int MAX = 8;
+  int n = 0;
+  unsigned* p[MAX];
+  size_t words[MAX];
+  template <typename T>
+  void add(T* q, size_t count) {
+    static_assert(sizeof(T) % 4 == 0, "words");
+    p[n] = reinterpret_cast<unsigned*>(q);
+    words[n++] = count * (sizeof(T) / 4);
+  }
+};
+cudaError_t launch_zero(const ZeroList& z, int num_sms, cudaStream_t s);
 // knots mc[n] reordered heaviest first by steps[knot] (quarter-octave groups)
 cudaError_t launch_lpt_order(const int* mc, int n, const unsigned long long* steps, int* out, cudaStream_t s);
 // Sets the Philox key schedule (rk) of `seed` and the instance word.
