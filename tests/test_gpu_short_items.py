@@ -25,3 +25,19 @@ def test_chosen_size(nsub, nnode, npaths, opts, threads):
             # FP32 sums of the same terms in another order (64 products at a time)
             np.testing.assert_allclose(a.val, b.val, rtol=0, atol=64 * 2.0 ** -24)
             np.testing.assert_allclose(a.B, b.B, rtol=0, atol=1e-6 * np.max(np.abs(a.B)))
+
+
+@pytest.mark.parametrize("circle", [False, True])
+def test_continuation_size(circle):
+    """Variance-adaptive paths: the continuation's own CTA size, the same paths."""
+    opts = dict(seed=6, adaptive_n=True, npaths_max=20_000, target_stderr=4e-3, richardson=True, adaptive_h=True)
+    pd = P.PDDSparseGM.circle_mesh(1.0, 3, 8, 7) if circle else \
+        P.PDDSparseGM((-1.0, -1.0), (1.0, 1.0), 3, 7, fac_rule(2.0, 3, 7))
+    with pd:
+        bvp = P.BVP.circle_poisson() if circle else P.BVP.poisson_sincos()
+        a = pd.estimate(bvp, 500, 2e-3, **opts)
+        b = pd.estimate(bvp, 500, 2e-3, cta_threads=256, **opts)
+        assert np.array_equal(a.npaths, b.npaths) and a.npaths.max() > 4096 + 500
+        assert a.info["path_steps"] == b.info["path_steps"]
+        # FP32 sums of the same terms in another order (64 products at a time)
+        np.testing.assert_allclose(a.val, b.val, rtol=0, atol=64 * 2.0 ** -24)
