@@ -1039,7 +1039,6 @@ pdds_status pdds_destroy(pdds_ctx* ctx) {
     ctx->sexch.recycle();
     ctx->fast64.recycle();
     ctx->fp64_S.recycle();
-    ctx->fp64_next.recycle();
     ctx->knot_rng.recycle();
     ctx->tab.recycle();
     ctx->lut_coef.recycle();
@@ -1518,10 +1517,7 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
       const int n_blocks = rn * chunks;
       a.sum_stride = std::max(ctx->fp64_nall, 1);
       CK(ctx->fp64_S.resize((size_t)std::max(n_blocks, 1) * FP64_SLOTS * a.sum_stride));
-      CK(ctx->fp64_next.resize(std::max(n_blocks, 1)));
-      CK(cudaMemsetAsync(ctx->fp64_next.p, 0, std::max(n_blocks, 1) * sizeof(int), s));
       a.S = ctx->fp64_S.p;
-      a.next_path = ctx->fp64_next.p;
       // a CTA takes a whole block (its lanes share the block's paths and the
       // stencil's set-up) unless that leaves SMs without work: 19 blocks of
       // one knot's 5,000 paths take 0.67 ms as 19 CTAs, 0.49 ms as 152
@@ -1531,7 +1527,8 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
       const size_t smem = (size_t)(slots + 1) * a.sum_stride * sizeof(double);
       const int bps = std::max(1, fp64_blocks_per_sm(P.kind, smem, a.richardson, threads));
       a.n_items = n_blocks * (FP64_SLOTS / slots);
-      const int grid = std::max(1, std::min(a.n_items, bps * ctx->num_sms));
+      a.spread = slots < FP64_SLOTS ? 1 : 0;
+      const int grid = a.spread ? a.n_items : std::max(1, std::min(a.n_items, bps * ctx->num_sms));
       if (a.n_items > 0) {
         CK(launch_paths_fp64(a, P.kind, grid, threads, smem, s));
         CK(launch_rows_fp64(a, n_blocks, s));

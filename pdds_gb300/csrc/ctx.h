@@ -245,7 +245,6 @@ struct pdds_ctx {
   DBuf<unsigned char> fast64;     // tables of the FP64 path kernel, filled by the first FP64 estimate
   bool fast64_ready = false;
   DBuf<double> fp64_S;            // RBF sums of the FP64 path kernel
-  DBuf<int> fp64_next;            // and its blocks' path counters
   DBuf<int> mc_lpt;               // MIXED hand-out order, heaviest knots first (from knot_steps)
   bool lpt_ready = false;
   bool has_knot_steps = false;

@@ -2,7 +2,8 @@
 //
 // The paths of a knot are split into blocks of block_paths; a block is eight
 // slots of 32 lanes, slot w starting with the block's paths [32 w, 32 w + 32)
-// and every lane taking the block's next path when its own ends.  Every path
+// and every lane taking one of the block's further paths when its own ends,
+// by a rule on step counts alone.  Every path
 // quantity is FP64 and each stencil exit adds its exact RBF vector
 // Y * r_j(X), r_j = exp(-|p_j - X|^2 / c^2), into the FP64 sums S_j of its
 // slot.  Afterwards (k_rows_fp64) G_i = -(1/N) sum_j ipsi(j,i) S_j per block.
@@ -21,13 +22,20 @@
 // the sums of B come from tables (fast64.cuh); the exit test of
 // constant-sigma kinds compares |x - c| with an edge formed once, as
 // integers; the normals of odd and even steps come from one place, so lanes
-// of both kinds do not run it twice.  What reaches the sums S keeps its
-// rounding and its order (positions, exponentials, the slots' sums): Psi^-1
-// has entries of 1e9 and more, so G carries the rounding of S and of the
-// product with it, and another grouping of the paths moves G by more than
-// the Monte Carlo noise of two runs.
-// 4x4/n11, N = 1e4, h = 1e-3: 49.7 -> 24.8 ms; one knot of 5,000 paths
+// of both kinds do not run it twice.  Positions, exponentials and the order
+// in which a slot's exits are added have to stay: Psi^-1 has entries of 1e9
+// and more, so G carries the rounding of the sums S.  A path that enters
+// another slot's sum moves G by 1e-8 to 1e-5 of its size (one knot of 5,000
+// paths: 1.3e-6 in the median over 40
+// seeds), which is why the hand-out may not depend on which warp comes first.
+// With an atomic counter in its place, two runs on the same inputs put 35 %
+// of the further paths into different slots; the exchange that replaces it
+// costs nothing for one knot (742 against 747 us for the whole call) and
+// 1.7 % at 4x4/n11.
+// 4x4/n11, N = 1e4, h = 1e-3: 49.7 -> 25.2 ms; one knot of 5,000 paths
 // 1.02 -> 0.49 ms.
+#include <cooperative_groups.h>
+
 #include "dev_common.cuh"
 #include "fast64.cuh"
 #include "kernels.h"
@@ -152,6 +160,7 @@ k_paths_fp64(const Fp64Args a) {
   __shared__ ItemSide64 s_side[4];
   __shared__ double s_rect[4];
   __shared__ int s_item, s_knot, s_nall;
+  __shared__ unsigned s_ends[2][FP64_SLOTS];  // slots: ends in this iteration, and iterations with ends before
   __shared__ double s_h;
   __shared__ double s_red[FP64_THREADS / 32][2];
   __shared__ double s_diag[PDDS_DIAG_N];
@@ -159,9 +168,11 @@ k_paths_fp64(const Fp64Args a) {
   const DevLayout& L = a.L;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nthr = blockDim.x, NW = nthr >> 5;  // NW slots of a block
+  const unsigned lt = (1u << lane) - 1u;
 
   for (;;) {
-    if (tid == 0) s_item = atomicAdd(a.item_counter, 1);
+    // blocks spread over CTAs: one item per CTA, a block's CTAs next to each other
+    if (tid == 0) s_item = a.spread ? (int)blockIdx.x : atomicAdd(a.item_counter, 1);
     __syncthreads();
     const int item = s_item;
     if (item >= a.n_items) break;
@@ -169,7 +180,7 @@ k_paths_fp64(const Fp64Args a) {
     const int groups = FP64_SLOTS / NW;
     const int block = item / groups, slot = (item - block * groups) * NW + warp;
     const int kn = block / a.blocks, p0 = (block - kn * a.blocks) * a.block_paths;
-    const int path_end = min(a.N, p0 + a.block_paths);
+    const unsigned path_end = (unsigned)min((int64_t)a.N, (int64_t)p0 + a.block_paths);
     if (tid == 0) {
       const int k = a.mc_knots[kn];
       s_knot = k;
@@ -248,7 +259,21 @@ k_paths_fp64(const Fp64Args a) {
     Coef<double> k0;
     if constexpr (!iso64<KIND>) coef_t64<KIND>(a.P, T, x0, y0, k0);
     unsigned path = (unsigned)(p0 + 32 * slot + lane);
-    bool active = (int)path < path_end;
+    bool active = path < path_end;
+    // Hand-out of the block's paths beyond the slots' first ones: by the
+    // iteration in which a lane's path ends, then the slot with fewer such
+    // iterations so far, the higher slot, the lower lane.  A path's slot
+    // decides which of the sums S its exits enter, so no timing may enter
+    // here; while paths are left (every lane of the block then has one) the
+    // block's warps exchange their ends after every iteration.  The rule is
+    // the order in which the warps of one CTA come to an atomic counter,
+    // nearly: of 22,261 hand-outs to two slots in one iteration 1,178 came
+    // first to the one with fewer ends and 52 to the other.
+    unsigned next = (unsigned)p0 + 32u * FP64_SLOTS;  // next path to hand out, the same in every warp
+    unsigned ends = 0;                                // iterations of this slot with ends
+    unsigned phase = 0;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    if (a.spread && next < path_end) cluster.sync();  // every CTA of the block has started
     double b = 0.0, bb = 0.0;
     unsigned long long nsteps = 0, nglob = 0, nsten = 0;
     // exit on side d at side coordinate `along` (x or y on rectangles, angle
@@ -446,8 +471,8 @@ k_paths_fp64(const Fp64Args a) {
     u32x4 blk;
     blk.v[0] = blk.v[1] = blk.v[2] = blk.v[3] = 0;
     while (__any_sync(FULL, active)) {
+      bool fin = false;  // the lane's path (pair) finished in this iteration
       if (active) {
-        bool fin = false;  // the lane's path (pair) finished in this iteration
         if (RICH) {
           const unsigned mi = m++;
           blk = path_block(a.seed, a.instance, knot_word(a.L, knot), path, mi);
@@ -494,16 +519,35 @@ k_paths_fp64(const Fp64Args a) {
             if (a.diag) diag_add(s_diag, fine.phi, fine.xi, fine.steps * h, 2.0 * fine.steps);
           }
         }
-        if (fin) {
-          path = (unsigned)(p0 + 32 * FP64_SLOTS) + (unsigned)atomicAdd(a.next_path + block, 1);
-          if ((int)path >= path_end) {
-            active = false;
-          } else {
-            reset();
-            fine_alive = true;
-            coarse_alive = RICH;
-            m = 0;
-          }
+      }
+      const unsigned fm = __ballot_sync(FULL, fin);
+      unsigned take = path_end;
+      if (next < path_end) {
+        const unsigned mine = (unsigned)__popc(fm) | ends << 8;
+        unsigned* slots = s_ends[phase];
+        if (a.spread) {
+          if (lane < groups) *cluster.map_shared_rank(slots + slot, lane) = mine;
+          cluster.sync();
+        } else {
+          if (lane == 0) slots[slot] = mine;
+          __syncthreads();
+        }
+        const unsigned other = lane < FP64_SLOTS ? slots[lane] : 0u, n = other & 0xffu;
+        const bool first = other >> 8 < ends || (other >> 8 == ends && lane > slot);
+        take = next + __reduce_add_sync(FULL, first ? n : 0u) + (unsigned)__popc(fm & lt);
+        next += __reduce_add_sync(FULL, n);
+        ends += fm != 0u;
+        phase ^= 1u;
+      }
+      if (fin) {
+        path = take;
+        if (path >= path_end) {
+          active = false;
+        } else {
+          reset();
+          fine_alive = true;
+          coarse_alive = RICH;
+          m = 0;
         }
       }
       flush(32);
@@ -545,6 +589,7 @@ k_paths_fp64(const Fp64Args a) {
       atomicAdd(a.stats + 3, tt);
     }
     if (a.diag) diag_flush(s_diag, a.diag + (int64_t)knot * PDDS_DIAG_N, tid);
+    if (a.spread) break;
     __syncthreads();
   }
 }
@@ -607,8 +652,19 @@ static cudaError_t launch_fp64_t(const Fp64Args& a, int kind, int grid, int thre
 #define PDDS_FP64_CASE(KK, GG)                                                                           \
   case KK:                                                                                               \
     cudaFuncSetAttribute(k_paths_fp64<KK, RICH, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    k_paths_fp64<KK, RICH, GG><<<grid, threads, smem, s>>>(a);                                      \
-    break;
+    return cudaLaunchKernelEx(&cfg, k_paths_fp64<KK, RICH, GG>, a);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  // the CTAs of a spread block exchange their ends through distributed shared memory
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = (unsigned)(FP64_SLOTS * 32 / threads);
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = a.spread ? 1 : 0;
   if (a.L.geom == 1) {
     switch (kind) {
       PDDS_FP64_CASE(0, 1)
@@ -628,7 +684,6 @@ static cudaError_t launch_fp64_t(const Fp64Args& a, int kind, int grid, int thre
     }
   }
 #undef PDDS_FP64_CASE
-  return cudaGetLastError();
 }
 
 cudaError_t launch_paths_fp64(const Fp64Args& a, int kind, int grid, int threads, size_t smem, cudaStream_t s) {

@@ -145,7 +145,7 @@ struct Fp64Args {
   long long max_steps;
   const int* mc_knots;
   int* item_counter;
-  int* next_path;           // per block, zeroed: paths handed out beyond the slots' first ones
+  int spread;               // 1: a block takes a cluster of CTAs, one item per CTA
   double* S;                // [knots x blocks][FP64_SLOTS][sum_stride]: the slots' RBF sums
   int sum_stride;
   double* G;
