@@ -281,6 +281,10 @@ pdds_status pdds_batch_run(pdds_ctx* ctx, const pdds_batch_run_desc* desc, pdds_
     if (st != PDDS_OK) return st;
   }
   if (desc->waves < 0) return fail(ctx, PDDS_ERR_INVALID, "waves must be >= 0");
+  {
+    const pdds_status st = check_hist_smem(ctx, &ed);
+    if (st != PDDS_OK) return st;
+  }
   if (!ctx->solve_stream) {
     int least = 0, greatest = 0;
     CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -335,6 +339,7 @@ pdds_status pdds_batch_run(pdds_ctx* ctx, const pdds_batch_run_desc* desc, pdds_
   std::memcpy(key.data() + sizeof(pdds_batch_run_desc) + sizeof(int), after, sizeof(after));
   int launches = 0;
   bool replayed = false;
+  const SetupGuard guard(ctx);
   if (desc->use_graph) {
     if (!ctx->graph_exec || ctx->graph_key != key) {
       drop_graph(ctx);

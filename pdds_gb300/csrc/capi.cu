@@ -474,13 +474,16 @@ pdds_status join_setup(pdds_ctx* ctx) {
   return PDDS_OK;
 }
 
+SetupGuard::~SetupGuard() {
+  if (!ctx->setup_pending) return;
+  cudaStreamSynchronize(ctx->setup_stream);
+  ctx->setup_pending = false;
+  ctx->tables_ready = false;
+}
+
 pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const ProblemDev& P, bool events,
                            int* launches) {
   cudaStream_t s = ctx->stream;
-  {  // tables of an earlier call that failed before its contraction
-    const pdds_status st = join_setup(ctx);
-    if (st != PDDS_OK) return st;
-  }
   HostLayout& L = ctx->L;
   const int mode = desc->mode;
   const int64_t nnz = L.row_ptr[L.K];
@@ -518,14 +521,12 @@ pdds_status enqueue_prefix(pdds_ctx* ctx, const pdds_estimate_desc* desc, const 
       sr = ctx->setup_stream;
       CK(cudaEventRecord(ctx->setup_ev[0], s));
       CK(cudaStreamWaitEvent(sr, ctx->setup_ev[0], 0));
+      ctx->setup_pending = true;
     }
     CK(launch_rbf_setup(ctx->dl, ctx->max_n, ctx->max_nbins, ctx->ipsi.p, ctx->tab.p, ctx->rbf_lu.p, ctx->rbf_piv.p,
                         ctx->rbf_uinv.p, ctx->errf.p, sr));
     *launches += 4;
-    if (sr != s) {
-      CK(cudaEventRecord(ctx->setup_ev[1], sr));
-      ctx->setup_pending = true;
-    }
+    if (sr != s) CK(cudaEventRecord(ctx->setup_ev[1], sr));
     ctx->tables_ready = true;
   }
   if (events) CK(cudaEventRecord(ctx->ev1, s));
@@ -673,6 +674,14 @@ bool short_items(const pdds_ctx* ctx, const MixedArgs& a, int mk, int n_items, i
   return lanes(128) >= lanes(256);
 }
 
+constexpr size_t MIXED_SMEM_CAP = 200 * 1024;  // dynamic shared memory of a path-kernel CTA
+pdds_status hist_refused(pdds_ctx* ctx) {
+  return fail(ctx, PDDS_ERR_INVALID, "exit histograms exceed shared memory; lower bins_per_gap");
+}
+size_t hist_smem(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int threads) {
+  return ctx->mixed_smem * (desc->want_var ? 2 : 1) + mixed_queue_smem(threads, desc->richardson ? 1 : 0);
+}
+
 pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, const ProblemDev& P, int chunks,
                                 int ppc, int* launches, const ItemList* items = nullptr, int mc0 = 0,
                                 int mc_n = -1, const int* order = nullptr) {
@@ -779,7 +788,7 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   if (!items && desc->cta_threads == 0 && !tuned_for(ctx, desc) && short_items(ctx, a, mk, n_items, ppc, threads))
     threads = 128;
   if (!items) ctx->run_threads = threads;
-  const size_t base_smem = ctx->mixed_smem * (a.want_var ? 2 : 1) + mixed_queue_smem(threads, a.richardson);
+  const size_t base_smem = hist_smem(ctx, desc, threads);
   a.hist_cap = (int)(ctx->mixed_smem / sizeof(float));
   a.hist_stride = slot_words(ctx, desc);
   a.var_off = hist_words(ctx);
@@ -788,7 +797,7 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   a.mc_pos = ctx->mc_pos.p;
   a.mc0 = mc0;
   const size_t smem = base_smem + (mk == PK_LUT ? lut_stage(ctx, P, base_smem, threads, &a.lut_nodes) : 0);
-  if (smem > 200 * 1024) return fail(ctx, PDDS_ERR_INVALID, "exit histograms exceed shared memory; lower bins_per_gap");
+  if (smem > MIXED_SMEM_CAP) return hist_refused(ctx);
   int bps = mixed_blocks_per_sm(mk, smem, a.richardson, threads, a.diag != nullptr);
   if (bps < 1) bps = 1;
   if (ctx->force_bps > 0) bps = std::min(bps, ctx->force_bps);
@@ -915,6 +924,11 @@ pdds_status adaptive_continue(pdds_ctx* ctx, const pdds_estimate_desc* desc, con
     if (st != PDDS_OK) return st;
   }
   return PDDS_OK;
+}
+
+pdds_status check_hist_smem(pdds_ctx* ctx, const pdds_estimate_desc* desc) {
+  const int threads = desc->cta_threads > 0 ? desc->cta_threads : 128;  // the smaller size, if both may come
+  return hist_smem(ctx, desc, threads) > MIXED_SMEM_CAP ? hist_refused(ctx) : PDDS_OK;
 }
 
 pdds_status order_groups(pdds_ctx* ctx, const pdds_estimate_desc* desc, const std::vector<int>& first) {
@@ -1378,17 +1392,22 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
   const ProblemDev P = problem_dev(ctx);
   const int N = desc->npaths;
   int launches = 0;
-  ctx->run_threads = cta_threads_for(ctx, desc);
-  {
-    pdds_status st = enqueue_prefix(ctx, desc, P, true, &launches);
-    if (st != PDDS_OK) return st;
-  }
   const int n_mc = ctx->n_mc;
   // the hand-out positions this call runs
   const int r0 = desc->knot_first;
   const int rn = desc->knot_count > 0 ? desc->knot_count : n_mc - r0;
   if (r0 > n_mc || (int64_t)r0 + rn > n_mc)
     return fail(ctx, PDDS_ERR_INVALID, "knot range beyond the layout's " + std::to_string(n_mc) + " knots with paths");
+  if (mode == PDDS_MODE_MIXED) {
+    const pdds_status st = check_hist_smem(ctx, desc);
+    if (st != PDDS_OK) return st;
+  }
+  ctx->run_threads = cta_threads_for(ctx, desc);
+  const SetupGuard guard(ctx);
+  {
+    pdds_status st = enqueue_prefix(ctx, desc, P, true, &launches);
+    if (st != PDDS_OK) return st;
+  }
   if (mode == PDDS_MODE_REPLAY_FP64) {
     const int64_t total = (int64_t)rn * N;
     CK(ctx->rx.resize(std::max<int64_t>(total, 1)));
@@ -1624,7 +1643,10 @@ pdds_status pdds_autotune(pdds_ctx* ctx, const pdds_estimate_desc* desc, int32_t
   pdds_estimate_desc d = *desc;
   d.adaptive_n = 0;
   int launches = 0;
-  pdds_status st = enqueue_prefix(ctx, &d, P, false, &launches);
+  pdds_status st = check_hist_smem(ctx, &d);
+  if (st != PDDS_OK) return st;
+  const SetupGuard guard(ctx);
+  st = enqueue_prefix(ctx, &d, P, false, &launches);
   if (st == PDDS_OK) st = join_setup(ctx);
   if (st != PDDS_OK) return st;
   // a block size imposed by the caller is kept: only the other shape

@@ -272,6 +272,19 @@ pdds_status enqueue_mixed(pdds_ctx* ctx, const pdds_estimate_desc* desc, int* la
 pdds_status order_groups(pdds_ctx* ctx, const pdds_estimate_desc* desc, const std::vector<int>& first);
 // Makes ctx->stream wait for the tables of this call's prefix.
 pdds_status join_setup(pdds_ctx* ctx);
+// Held by every call that runs a prefix: when the call returns before its
+// join (it failed in between), the host waits for the set-up work.  The next
+// call may replace the layout that this work reads and writes, and only
+// ctx->stream is waited for, or ordered, there.
+struct SetupGuard {
+  pdds_ctx* ctx;
+  explicit SetupGuard(pdds_ctx* c) : ctx(c) {}
+  SetupGuard(const SetupGuard&) = delete;
+  ~SetupGuard();
+};
+// PDDS_ERR_INVALID if no CTA size that the estimate may run with has room for
+// its exit histograms (asked before anything is launched).
+pdds_status check_hist_smem(pdds_ctx* ctx, const pdds_estimate_desc* desc);
 // Words of exit histograms that enqueue_mixed needs for mc_n knots.
 size_t mixed_hist_words(const pdds_ctx* ctx, const pdds_estimate_desc* desc, int mc_n);
 // Destroys the captured batch graph (its kernels hold buffer addresses).
