@@ -4,7 +4,7 @@
 // weights.
 //
 // Counterpart of the reference's per-exit loop over the side's RBF centres
-// (PDDAlgorithms/PDDSparseGM.cpp, Update_G); the path kernel used to do this
+// (G_update, Meshes/stencil.cpp:244-307); the path kernel used to do this
 // at the end of each work item, with its own 128 or 256 threads.
 //
 // What bounds it: instruction issue (60 % at 12x12/n43), of FMAs to a third.
@@ -22,8 +22,8 @@
 // with variances 3.50 -> 3.42.
 //
 // Rounding is that of the loop it replaces: FP32 sums of 64 products in the
-// same order for each item, added in two floats (TwoSum, 48 bits; FP64 issues
-// at 1/64 of the rate) and over the items in FP64.  Adding a knot's items
+// same order for each item, added to more than FP64 accuracy in three floats
+// (pair_sum.cuh) and over the items in FP64.  Adding a knot's items
 // before the products would save 0.04 of 3.42 ms at 741 knots, but the
 // products' rounding would not average over the items.
 #include <cuda_runtime.h>
@@ -32,6 +32,7 @@
 
 #include "dev_common.cuh"
 #include "kernels.h"
+#include "pair_sum.cuh"
 
 namespace pdds {
 
@@ -53,19 +54,6 @@ __device__ __forceinline__ void copy4(float* dst, const float* src, bool in) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
                "r"(in ? 4 : 0)
                : "memory");
-}
-
-// s + e exactly (e the running error), two sums at once: TwoSum
-__device__ __forceinline__ void add2(float2& s, float2& e, float2 v) {
-  auto sub = [](float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); };
-  const float2 t = __fadd2_rn(s, v), b = sub(t, s);
-  e = __fadd2_rn(e, __fadd2_rn(sub(s, sub(t, b)), sub(v, b)));
-  s = t;
-}
-// one of the two; an infinite sum has no error term
-__device__ __forceinline__ double total(float2 s2, float2 e2, int second) {
-  const float s = second ? s2.y : s2.x, e = second ? e2.y : e2.x;
-  return (double)s + (isfinite(s) ? (double)e : 0.0);
 }
 
 struct RowInfo {
@@ -102,14 +90,18 @@ __device__ __forceinline__ void contract_columns(const ContractArgs& a, const Ro
   // rows in pairs: one instruction for two products
   constexpr int RP = RT / 2;
   const float2 zero = make_float2(0.f, 0.f);
-  float2 hi[RP][NJ], lo[RP][NJ], p[RP][NJ];
-  float2 hi2[VAR ? RP : 1][NJ], lo2[VAR ? RP : 1][NJ], p2[VAR ? RP : 1][NJ];
+  PairSum sum[RP][NJ], sum2[VAR ? RP : 1][NJ];
+  float2 p[RP][NJ], p2[VAR ? RP : 1][NJ];
 #pragma unroll
   for (int r = 0; r < RP; r++)
 #pragma unroll
     for (int j = 0; j < NJ; j++) {
-      hi[r][j] = lo[r][j] = p[r][j] = zero;
-      if (VAR) hi2[r][j] = lo2[r][j] = p2[r][j] = zero;
+      p[r][j] = zero;
+      sum[r][j] = {zero, zero, zero};
+      if (VAR) {
+        p2[r][j] = zero;
+        sum2[r][j] = {zero, zero, zero};
+      }
     }
   auto issue = [&](int st) {
     if (st < st1) {
@@ -179,10 +171,10 @@ __device__ __forceinline__ void contract_columns(const ContractArgs& a, const Ro
       for (int r = 0; r < RP; r++)
 #pragma unroll
         for (int j = 0; j < NJ; j++) {
-          add2(hi[r][j], lo[r][j], p[r][j]);
+          pair_add(sum[r][j], p[r][j]);
           p[r][j] = zero;
           if (VAR) {
-            add2(hi2[r][j], lo2[r][j], p2[r][j]);
+            pair_add(sum2[r][j], p2[r][j]);
             p2[r][j] = zero;
           }
         }
@@ -204,8 +196,8 @@ __device__ __forceinline__ void contract_columns(const ContractArgs& a, const Ro
       if (!a.dup_sum && !a.L.map_owner[m]) continue;
       const int64_t e = a.L.map_pos[m];
       if (!idx_ok(e, a.L.row_ptr[ri.knot + 1] - ri.e0, a.err_flags)) continue;
-      atomicAdd(a.G + ri.e0 + e, -total(hi[r / 2][j], lo[r / 2][j], r & 1) * invN);
-      if (VAR) atomicAdd(a.GG + ri.e0 + e, total(hi2[r / 2][j], lo2[r / 2][j], r & 1) * invN);
+      atomicAdd(a.G + ri.e0 + e, -pair_total(sum[r / 2][j], r & 1) * invN);
+      if (VAR) atomicAdd(a.GG + ri.e0 + e, pair_total(sum2[r / 2][j], r & 1) * invN);
     }
   }
 }
