@@ -926,6 +926,9 @@ pdds_status adaptive_continue(pdds_ctx* ctx, const pdds_estimate_desc* desc, con
   return PDDS_OK;
 }
 
+// Device memory for the slots' RBF sums of one FP64 launch.
+constexpr int64_t FP64_MAX_BYTES = int64_t(512) << 20;
+
 pdds_status check_hist_smem(pdds_ctx* ctx, const pdds_estimate_desc* desc) {
   const int threads = desc->cta_threads > 0 ? desc->cta_threads : 128;  // the smaller size, if both may come
   return hist_smem(ctx, desc, threads) > MIXED_SMEM_CAP ? hist_refused(ctx) : PDDS_OK;
@@ -1523,7 +1526,6 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
       a.adaptive_h = desc->adaptive_h ? 1 : 0;
       a.richardson = desc->richardson ? 1 : 0;
       a.max_steps = max_steps;
-      a.mc_knots = ctx->mc_knots.p + r0;
       a.item_counter = ctx->counter.p;
       a.G = ctx->G.p;
       a.Bsum = ctx->Bsum.p;
@@ -1533,22 +1535,28 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
       a.diag = diag ? ctx->diag.p : nullptr;
       a.blocks = chunks;
       a.block_paths = ppc;
-      const int n_blocks = rn * chunks;
       a.sum_stride = std::max(ctx->fp64_nall, 1);
-      CK(ctx->fp64_S.resize((size_t)std::max(n_blocks, 1) * FP64_SLOTS * a.sum_stride));
+      // the blocks' sums: the knots of one launch after another's where they
+      // take more than FP64_MAX_BYTES (10,945 knots of 12x12/n43: 256 MB)
+      const int64_t knot_words = (int64_t)chunks * FP64_SLOTS * a.sum_stride;
+      const int part = (int)std::max<int64_t>(1, std::min<int64_t>(rn, FP64_MAX_BYTES / 8 / knot_words));
+      CK(ctx->fp64_S.resize((size_t)part * knot_words));
       a.S = ctx->fp64_S.p;
-      // a CTA takes a whole block (its lanes share the block's paths and the
-      // stencil's set-up) unless that leaves SMs without work: 19 blocks of
-      // one knot's 5,000 paths take 0.67 ms as 19 CTAs, 0.49 ms as 152
-      int slots = FP64_SLOTS;
-      while (slots > 1 && n_blocks * (FP64_SLOTS / slots) < 2 * ctx->num_sms) slots /= 2;
-      const int threads = 32 * slots;
-      const size_t smem = (size_t)(slots + 1) * a.sum_stride * sizeof(double);
-      const int bps = std::max(1, fp64_blocks_per_sm(P.kind, smem, a.richardson, threads));
-      a.n_items = n_blocks * (FP64_SLOTS / slots);
-      a.spread = slots < FP64_SLOTS ? 1 : 0;
-      const int grid = a.spread ? a.n_items : std::max(1, std::min(a.n_items, bps * ctx->num_sms));
-      if (a.n_items > 0) {
+      for (int m = 0; m < rn; m += part) {
+        const int n_blocks = std::min(part, rn - m) * chunks;
+        a.mc_knots = ctx->mc_knots.p + r0 + m;
+        // a CTA takes a whole block (its lanes share the block's paths and the
+        // stencil's set-up) unless that leaves SMs without work: 19 blocks of
+        // one knot's 5,000 paths take 0.67 ms as 19 CTAs, 0.49 ms as 152
+        int slots = FP64_SLOTS;
+        while (slots > 1 && n_blocks * (FP64_SLOTS / slots) < 2 * ctx->num_sms) slots /= 2;
+        const int threads = 32 * slots;
+        const size_t smem = (size_t)(slots + 1) * a.sum_stride * sizeof(double);
+        const int bps = std::max(1, fp64_blocks_per_sm(P.kind, smem, a.richardson, threads));
+        a.n_items = n_blocks * (FP64_SLOTS / slots);
+        a.spread = slots < FP64_SLOTS ? 1 : 0;
+        const int grid = a.spread ? a.n_items : std::min(a.n_items, bps * ctx->num_sms);
+        if (m > 0) CK(cudaMemsetAsync(ctx->counter.p, 0, sizeof(int), s));
         CK(launch_paths_fp64(a, P.kind, grid, threads, smem, s));
         CK(launch_rows_fp64(a, n_blocks, s));
         launches += 2;

@@ -48,3 +48,22 @@ def test_single_knot_repeats():
         # 19 blocks of paths, added into the row in any order: a block's sum is rounded 18 times
         for g in got[1:]:
             assert np.max(np.abs(g - got[0])) <= 19 * 2.0 ** -53 * np.max(np.abs(got[0])) * 19
+
+
+def test_launches_split_where_the_sums_need_more_memory():
+    # 31,597 knots, 23 KB of sums each: two launches; a quarter of the knots fits one
+    nsub, nnode = 20, 43
+    with P.PDDSparseGM((-1.0, -1.0), (1.0, 1.0), nsub, nnode, fac_rule(2.0, nsub, nnode)) as pd:
+        run = lambda first, count: pd.estimate(P.BVP.poisson_sincos(), 300, 2e-3, mode=P.MODE_FP64, seed=5,  # noqa: E731
+                                               knot_first=first, knot_count=count)
+        run(0, 1)  # a context's first FP64 call also fills its tables
+        a = run(0, 0)
+        n_mc = int(np.count_nonzero(a.npaths))
+        bounds = [n_mc * q // 4 for q in range(5)]
+        parts = [run(lo, hi - lo) for lo, hi in zip(bounds, bounds[1:])]
+        assert a.info["kernel_launches"] == parts[0].info["kernel_launches"] + 2
+        assert np.array_equal(a.val, sum(p.val for p in parts))  # a row is zero outside its part
+        interior = a.npaths > 0
+        np.testing.assert_allclose(a.B[interior], sum(np.where(p.npaths > 0, p.B, 0.0) for p in parts)[interior],
+                                   rtol=0, atol=1e-12)
+        assert a.info["path_steps"] == sum(p.info["path_steps"] for p in parts)
