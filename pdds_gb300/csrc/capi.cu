@@ -935,13 +935,16 @@ pdds_status check_hist_smem(pdds_ctx* ctx, const pdds_estimate_desc* desc) {
 }
 
 pdds_status order_groups(pdds_ctx* ctx, const pdds_estimate_desc* desc, const std::vector<int>& first) {
-  if (first == ctx->lpt_groups) return PDDS_OK;
+  const bool adaptive = desc->adaptive_h != 0;
+  if (first == ctx->lpt_groups && desc->h == ctx->lpt_h && adaptive == ctx->lpt_adaptive) return PDDS_OK;
   std::vector<int> all;
   all.reserve(ctx->n_mc);
   for (size_t g = 0; g + 1 < first.size(); g++)
     for (int v : geometric_order(ctx, desc, first[g], first[g + 1] - first[g])) all.push_back(v);
   CK(ctx->mc_lpt.upload(all, ctx->stream));
   ctx->lpt_groups = first;
+  ctx->lpt_h = desc->h;
+  ctx->lpt_adaptive = adaptive;
   return PDDS_OK;
 }
 

@@ -185,7 +185,11 @@ struct pdds_ctx {
     int i0 = 0, m = 0;
     std::vector<pdds::ResidentPlan> plans;
   } batch_tail;
-  std::vector<int> lpt_groups;  // group bounds (hand-out positions) that mc_lpt is sorted for
+  // what mc_lpt is sorted for in a batch: group bounds (hand-out positions)
+  // and the step that the ranking uses
+  std::vector<int> lpt_groups;
+  double lpt_h = 0.0;
+  bool lpt_adaptive = false;
   int solve_m = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   // MIXED: the RBF factorisation and tables run beside the paths, which do
