@@ -415,8 +415,9 @@ typedef struct {
   int32_t max_refine;    /* FP64 refinement steps */
   double tol;            /* relative residual in FP64 */
   /* GMRES over the whole GPU (systems of 4096 knots and more): polls of a
-   * grid-barrier wait before it gives up and the solve returns
-   * PDDS_ERR_TIMEOUT (0 = 2^24, about a second; >= 0) */
+   * wait between its CTAs before it gives up and the solve returns
+   * PDDS_ERR_TIMEOUT (0 = about a second: 2^24 polls of the grid barrier, or
+   * 2^21 where the system's rows fit on chip; >= 0) */
   int32_t barrier_poll_limit;
   /* PDDS_SOLVE_GMRES_FP32_IR: PDDS_GMRES_PIPELINED (0, the default) keeps
    * G V beside the basis and applies each step's product to the not yet

@@ -461,7 +461,7 @@ pdds_status check_err_flags(pdds_ctx* ctx) {
   if (f & ERR_FLAG_EXIT_SIDE) return fail(ctx, PDDS_ERR_EXIT_SIDE, "an exit matched no stencil side");
   if (f & ERR_FLAG_SUB_NOCONV)
     return fail(ctx, PDDS_ERR_NOT_CONVERGED, "a subdomain solve missed its tolerance in 200 iterations");
-  if (f & ERR_FLAG_TIMEOUT) return fail(ctx, PDDS_ERR_TIMEOUT, "a grid barrier of the interface solve timed out");
+  if (f & ERR_FLAG_TIMEOUT) return fail(ctx, PDDS_ERR_TIMEOUT, "a wait between the CTAs of the interface solve ran out");
   if (f & ERR_FLAG_BOUNDS)
     return fail(ctx, PDDS_ERR_BOUNDS, "a device index check failed (checked build): an access was skipped");
   return PDDS_OK;
@@ -2058,7 +2058,9 @@ pdds_status pdds_solve_interface(pdds_ctx* ctx, const pdds_solve_desc* desc, dou
     a.inner_tol = 1e-6;
     a.out = ctx->sscal.p;
     a.err_flags = ctx->errf.p;
-    a.spin_limit = w.spin_limit;
+    // the limit is for GMRES over the whole GPU: other solves had no waits to
+    // run out, and take the default one, of about a second, here
+    a.spin_limit = !bicg && K >= GMRES_WHOLE_GPU_ROWS ? w.spin_limit : 0;
     CK(launch_resident(a, plan, rmeth, ctx->sexch.p, s));
     w.launches = 1;
     double out[2] = {0.0, 0.0};

@@ -533,7 +533,7 @@ cudaError_t solve_gmres_ir_cluster(const SolveCsr& A, const double* b, double* x
   const int n = A.K;
   if (m < 2 || m > GMRES_CLUSTER_MAX_M) return cudaSuccess;
   // large systems: the whole GPU with grid barriers; small ones: one cluster
-  int gb = (n >= 4096 && w.bar && w.gpart && w.err) ? gmres_grid_blocks(n) : 0;
+  int gb = (n >= GMRES_WHOLE_GPU_ROWS && w.bar && w.gpart && w.err) ? gmres_grid_blocks(n) : 0;
   if (gb > 0 && w.grid_ctas > 0) gb = std::min(gb, w.grid_ctas);
   const int cl = gb > 0 ? 0 : gmres_cluster_pick(n);
   if (gb <= 0 && cl <= 0) return cudaSuccess;

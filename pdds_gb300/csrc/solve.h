@@ -82,6 +82,11 @@ cudaError_t launch_stamp(unsigned long long* t, cudaStream_t s);
 // b[i] = (float)a[i]
 cudaError_t launch_to_f32(const double* a, float* b, int64_t n, cudaStream_t s);
 
+// Systems from this many rows on are GMRES's "over the whole GPU": the grid
+// kernel rather than one cluster where the system does not fit on chip, and
+// the caller's poll limit counts.
+constexpr int GMRES_WHOLE_GPU_ROWS = 4096;
+
 // One interface system with its rows resident on chip (k_resident.cu).
 // How the system is split: CTA c owns the rows [row0[c], row0[c + 1]), at
 // most `per`; cap_* are the largest CTA's entries (0: BiCGSTAB entries that stay in L2), column-list
