@@ -333,7 +333,10 @@ k_paths_fp64(const Fp64Args a) {
       if constexpr (iso64<KIND>) {
         Coef<double> k;
         coef_t64<KIND>(a.P, T, s.x, s.y, k);
-        const double d0 = __dmul_rn(S, i0), d1 = __dmul_rn(S, i1);
+        // Robin: the increment's product may be fused with the push along the
+        // normal below, which is the rounding that this step has always had
+        const double d0 = KIND == PK_ROBIN ? S * i0 : __dmul_rn(S, i0);
+        const double d1 = KIND == PK_ROBIN ? S * i1 : __dmul_rn(S, i1);
         const double gd = fma(k.g0, d0, k.g1 * d1);
         if constexpr (react64<KIND> || KIND == PK_ROBIN) {
           s.xi = fma(-s.Y, gd, s.xi);
@@ -397,7 +400,10 @@ k_paths_fp64(const Fp64Args a) {
         }
         double along, Ex = 0.0, Ey = 0.0;
         if (d <= 1) {
-          const double rel = ::atan2(pa0 * s.y - pa1 * s.x, pa0 * s.x + pa1 * s.y);
+          // (the roundings of both forms stated: left to the compiler, they depend on the code around)
+          const double sn = RICH ? __dsub_rn(__dmul_rn(pa0, s.y), __dmul_rn(pa1, s.x))
+                                 : fma(pa0, s.y, -__dmul_rn(pa1, s.x));
+          const double rel = ::atan2(sn, fma(pa0, s.x, __dmul_rn(pa1, s.y)));
           along = rect[1] + (has_rays ? ::fmin(::fmax(rel, 0.0), rect[3] - rect[1])
                                       : (rel < 0.0 ? rel + 6.283185307179586 : rel));
           ::sincos(along, &Ey, &Ex);
