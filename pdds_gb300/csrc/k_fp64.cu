@@ -150,8 +150,14 @@ __device__ __forceinline__ bool abs_below(double d, double edge) {
          (unsigned long long)__double_as_longlong(edge);
 }
 
+// Two CTAs per SM, except where the registers of one are needed (tables) and
+// for Robin problems: the blocks of knots with a reflecting side take several
+// times the steps of the others, and two of them on one SM end later than one
+// after the other on SMs that take the next block when they are done (324
+// knots in pairs, 500 paths: 14.3 to 16.9 ms with two, 12.0 with one; 1,500
+// paths, adaptive steps: 156 and 140; without pairs 9.3 and 9.9).
 template <int KIND, bool RICH, int GEOM>
-__global__ void __launch_bounds__(FP64_THREADS, is_lut_kind(KIND) ? 1 : 2)
+__global__ void __launch_bounds__(FP64_THREADS, is_lut_kind(KIND) || KIND == PK_ROBIN ? 1 : 2)
 k_paths_fp64(const Fp64Args a) {
   extern __shared__ double Ssum[];  // [warps][sum n] the slots' RBF sums, then [sum n] local t
   __shared__ double s_qs[FP64_THREADS / 32][FP64_QCAP], s_qy[FP64_THREADS / 32][FP64_QCAP];
