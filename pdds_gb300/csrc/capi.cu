@@ -1538,6 +1538,7 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
       a.diag = diag ? ctx->diag.p : nullptr;
       a.blocks = chunks;
       a.block_paths = ppc;
+      a.slots = std::min(FP64_SLOTS, (ppc + 31) / 32);
       a.sum_stride = std::max(ctx->fp64_nall, 1);
       // the blocks' sums: the knots of one launch after another's where they
       // take more than FP64_MAX_BYTES (10,945 knots of 12x12/n43: 256 MB)
@@ -1549,15 +1550,36 @@ pdds_status pdds_estimate(pdds_ctx* ctx, const pdds_estimate_desc* desc, double*
         const int n_blocks = std::min(part, rn - m) * chunks;
         a.mc_knots = ctx->mc_knots.p + r0 + m;
         // a CTA takes a whole block (its lanes share the block's paths and the
-        // stencil's set-up) unless that leaves SMs without work: 19 blocks of
-        // one knot's 5,000 paths take 0.67 ms as 19 CTAs, 0.49 ms as 152
+        // stencil's set-up) unless that leaves fewer than two CTAs per SM: 19
+        // blocks of one knot's 5,000 paths take 0.67 ms as 19 CTAs, 0.49 ms as
+        // 152; 225 blocks of 500 paths 14.7 ms whole, 7.2 spread (circle).
+        // Slots without paths get no CTA.  Table problems with half of the
+        // slots filled or less are spread below one CTA per SM only: the
+        // table's reads bound them, not the FP64 pipe (225 blocks of 100
+        // paths in pairs 10.4 ms whole, 13.5 spread; of 256 paths 19.5 and
+        // 20.0, 177 blocks 16.3 and 13.8).
         int slots = FP64_SLOTS;
-        while (slots > 1 && n_blocks * (FP64_SLOTS / slots) < 2 * ctx->num_sms) slots /= 2;
+        auto groups = [&]() { return (a.slots + slots - 1) / slots; };
+        const int want = P.kind == PK_LUT && 2 * a.slots <= FP64_SLOTS ? ctx->num_sms : 2 * ctx->num_sms;
+        while (slots > 1 && n_blocks * groups() < want) slots /= 2;
         const int threads = 32 * slots;
         const size_t smem = (size_t)(slots + 1) * a.sum_stride * sizeof(double);
-        const int bps = std::max(1, fp64_blocks_per_sm(P.kind, smem, a.richardson, threads));
-        a.n_items = n_blocks * (FP64_SLOTS / slots);
-        a.spread = slots < FP64_SLOTS ? 1 : 0;
+        int bps = std::max(1, fp64_blocks_per_sm(P.kind, smem, a.richardson, threads));
+        // One CTA per SM, although two fit, where the launch is shorter than
+        // two rounds of pairs: eight warps all but fill the FP64 pipe, and two
+        // long blocks on one SM end later than one after the other on SMs that
+        // take the next block when they are done.  182 to 612 blocks of 256
+        // paths or more, against pairs: circles 0.62 to 0.8 of the time below
+        // 304, 0.95 to 1.03 up to 608 and 1.03 to 1.05 beyond; squares 0.8 to
+        // 1.03 below 608, 1.0 to 1.12 beyond.  Robin problems at any length
+        // (1,620 blocks in pairs 140 ms, with two CTAs per SM 155).  Where
+        // half of the slots are empty, whose warps leave the pipe idle, other
+        // squares keep pairs (100 paths: 1.0 to 1.2 of the time with one).
+        const bool brief = n_blocks * groups() < 2 * bps * ctx->num_sms, filled = 2 * a.slots > FP64_SLOTS;
+        const bool mirror = P.kind == PK_ROBIN && (int)P.p[0] != 0;
+        if (filled ? brief || mirror : brief && (ctx->L.geom == 1 || mirror)) bps = 1;
+        a.n_items = n_blocks * groups();
+        a.spread = groups() > 1 ? 1 : 0;
         const int grid = a.spread ? a.n_items : std::min(a.n_items, bps * ctx->num_sms);
         if (m > 0) CK(cudaMemsetAsync(ctx->counter.p, 0, sizeof(int), s));
         CK(launch_paths_fp64(a, P.kind, grid, threads, smem, s));

@@ -150,14 +150,8 @@ __device__ __forceinline__ bool abs_below(double d, double edge) {
          (unsigned long long)__double_as_longlong(edge);
 }
 
-// Two CTAs per SM, except where the registers of one are needed (tables) and
-// for Robin problems: the blocks of knots with a reflecting side take several
-// times the steps of the others, and two of them on one SM end later than one
-// after the other on SMs that take the next block when they are done (324
-// knots in pairs, 500 paths: 14.3 to 16.9 ms with two, 12.0 with one; 1,500
-// paths, adaptive steps: 156 and 140; without pairs 9.3 and 9.9).
 template <int KIND, bool RICH, int GEOM>
-__global__ void __launch_bounds__(FP64_THREADS, is_lut_kind(KIND) || KIND == PK_ROBIN ? 1 : 2)
+__global__ void __launch_bounds__(FP64_THREADS, is_lut_kind(KIND) ? 1 : 2)
 k_paths_fp64(const Fp64Args a) {
   extern __shared__ double Ssum[];  // [warps][sum n] the slots' RBF sums, then [sum n] local t
   __shared__ double s_qs[FP64_THREADS / 32][FP64_QCAP], s_qy[FP64_THREADS / 32][FP64_QCAP];
@@ -183,7 +177,7 @@ k_paths_fp64(const Fp64Args a) {
     const int item = s_item;
     if (item >= a.n_items) break;
     // item = (block, group of NW slots); block = (knot, chunk of paths)
-    const int groups = FP64_SLOTS / NW;
+    const int groups = (a.slots + NW - 1) / NW;
     const int block = item / groups, slot = (item - block * groups) * NW + warp;
     const int kn = block / a.blocks, p0 = (block - kn * a.blocks) * a.block_paths;
     const unsigned path_end = (unsigned)min((int64_t)a.N, (int64_t)p0 + a.block_paths);
@@ -636,7 +630,8 @@ __global__ void __launch_bounds__(ROWS64_THREADS) k_rows_fp64(const Fp64Args a) 
   for (int i = tid; i < nall; i += ROWS64_THREADS) {
     double t = src[i];
 #pragma unroll
-    for (int w = 1; w < FP64_SLOTS; w++) t += src[w * a.sum_stride + i];
+    for (int w = 1; w < FP64_SLOTS; w++)
+      if (w < a.slots) t += src[w * a.sum_stride + i];
     S[i] = t;
   }
   __syncthreads();
@@ -670,13 +665,14 @@ static cudaError_t launch_fp64_t(const Fp64Args& a, int kind, int grid, int thre
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  // the CTAs of a spread block exchange their ends through distributed shared memory
+  // the CTAs of a spread block with paths to hand out (all of its slots are
+  // filled) exchange their ends through distributed shared memory
   cudaLaunchAttribute cluster{};
   cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = (unsigned)(FP64_SLOTS * 32 / threads);
+  cluster.val.clusterDim.x = (unsigned)(a.slots * 32 / threads);
   cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
   cfg.attrs = &cluster;
-  cfg.numAttrs = a.spread ? 1 : 0;
+  cfg.numAttrs = a.spread && a.block_paths > 32 * FP64_SLOTS ? 1 : 0;
   if (a.L.geom == 1) {
     switch (kind) {
       PDDS_FP64_CASE(0, 1)

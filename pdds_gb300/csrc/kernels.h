@@ -138,14 +138,15 @@ struct Fp64Args {
   uint64_t seed;
   uint32_t instance;
   int blocks, block_paths;  // blocks of paths per knot, paths per block
-  int n_items;              // knots x blocks x (FP64_SLOTS / slots per CTA)
+  int slots;                // slots of a block that have paths
+  int n_items;              // knots x blocks x (slots / slots per CTA)
   int dup_sum;
   int adaptive_h;
   int richardson;
   long long max_steps;
   const int* mc_knots;
   int* item_counter;
-  int spread;               // 1: a block takes a cluster of CTAs, one item per CTA
+  int spread;               // 1: a block takes several CTAs, one item per CTA
   double* S;                // [knots x blocks][FP64_SLOTS][sum_stride]: the slots' RBF sums
   int sum_stride;
   double* G;
