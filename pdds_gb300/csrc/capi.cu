@@ -654,6 +654,12 @@ std::vector<int> geometric_order(const pdds_ctx* ctx, const pdds_estimate_desc* 
   return ord;
 }
 
+// Lanes of path-kernel CTAs of `threads` that an SM holds.
+int lanes_per_sm(const pdds_ctx* ctx, int mk, int want_var, int richardson, bool diag, int threads) {
+  const size_t smem = ctx->mixed_smem * (want_var ? 2 : 1) + mixed_queue_smem(threads, richardson);
+  return threads * mixed_blocks_per_sm(mk, smem, richardson, threads, diag);
+}
+
 // Whether 256-thread CTAs, the default below 8,192 knots, are better halved
 // for items of ppc paths: at an item's end a CTA waits for the longest of its
 // lanes' paths, so short items (a few paths per lane) want fewer lanes each,
@@ -666,12 +672,8 @@ std::vector<int> geometric_order(const pdds_ctx* ctx, const pdds_estimate_desc* 
 bool short_items(const pdds_ctx* ctx, const MixedArgs& a, int mk, int n_items, int ppc, int threads) {
   if (threads != 256 || ctx->L.geom != 0 || mk == PK_LUT || mk == PK_LUT_TEX) return false;
   if (ppc > 1300 || 4 * (int64_t)n_items < 9 * 8 * (int64_t)ctx->num_sms) return false;
-  if (!a.richardson) return true;
-  auto lanes = [&](int th) {
-    const size_t smem = ctx->mixed_smem * (a.want_var ? 2 : 1) + mixed_queue_smem(th, a.richardson);
-    return th * mixed_blocks_per_sm(mk, smem, a.richardson, th, a.diag != nullptr);
-  };
-  return lanes(128) >= lanes(256);
+  return !a.richardson || lanes_per_sm(ctx, mk, a.want_var, a.richardson, a.diag != nullptr, 128) >=
+                              lanes_per_sm(ctx, mk, a.want_var, a.richardson, a.diag != nullptr, 256);
 }
 
 constexpr size_t MIXED_SMEM_CAP = 200 * 1024;  // dynamic shared memory of a path-kernel CTA
@@ -890,6 +892,12 @@ pdds_status adaptive_continue(pdds_ctx* ctx, const pdds_estimate_desc* desc, con
   }
   // work items heaviest knot first, so that no long item starts near the end
   std::stable_sort(cost.begin(), cost.end());
+  double all_steps = 0.0, item_steps = 0.0;  // of the continuation, and of its longest item
+  for (auto& c : cost) {
+    const int more = kn[c.second] - N0;
+    all_steps -= c.first;
+    item_steps = std::max(item_steps, -c.first * std::min(ppc, more) / more);
+  }
   std::vector<int> order;
   order.reserve(cost.size());
   for (auto& c : cost) order.push_back(c.second);
@@ -911,15 +919,22 @@ pdds_status adaptive_continue(pdds_ctx* ctx, const pdds_estimate_desc* desc, con
     CK(ctx->item_p1.upload(ip1, s));
     ItemList items{ctx->item_knot.p, ctx->item_p0.p, ctx->item_p1.p, (int)ik.size(), ctx->knot_invN.p, ik.data()};
     // The continuation's CTA size: the one that the autotuner timed, else 128
-    // threads whatever the layout (table kinds excepted, not measured): its
-    // items are many and go out heaviest first, so the launch's end weighs
-    // little and the wait for an item's longest path is over fewer lanes.
-    // Continuations at 256 against 128 threads: circles of 456 to 1,520 knots
-    // 10.4 -> 9.8, 37.8 -> 35.2, 286.6 -> 269.3 ms; squares of 225 to 3,501
-    // knots 0.92 to 1.0 of the time.
+    // threads (table kinds excepted, not measured) where the launch is as long
+    // as 1.5 of its longest items on every such CTA: an item then waits for its
+    // longest path over fewer lanes, and the launch's end weighs little.  In
+    // shorter launches one long item sets the end, and takes up to twice as
+    // long on half the lanes.  128 threads against 256, 60 to 3,325 knots, six
+    // problems, by that number: below 0.5 1.05 to 1.72 of the time, to 1 0.95
+    // to 1.32, to 1.5 0.92 to 1.24, to 2 0.91 to 1.03, to 3 0.92 to 0.98,
+    // beyond 0.89 to 0.96.  Not where shared memory leaves squares fewer lanes
+    // per SM (31 knots a side with variances in pairs 1.0 to 1.16; circles
+    // 0.95 all the same).
     pdds_estimate_desc dc = *desc;
     if (dc.cta_threads == 0 && tuned_for(ctx, desc)) dc.cta_threads = std::max(0, ctx->tune_cont_threads);
-    else if (dc.cta_threads == 0 && P.kind != PK_LUT) dc.cta_threads = 128;
+    else if (dc.cta_threads == 0 && P.kind != PK_LUT && all_steps >= 1.5 * 8.0 * ctx->num_sms * item_steps &&
+             (L.geom == 1 || lanes_per_sm(ctx, mixed_kind(P), dc.want_var, dc.richardson ? 1 : 0, false, 128) >=
+                                 lanes_per_sm(ctx, mixed_kind(P), dc.want_var, dc.richardson ? 1 : 0, false, 256)))
+      dc.cta_threads = 128;
     pdds_status st = enqueue_mixed_paths(ctx, &dc, P, 1, ppc, launches, &items);
     if (st != PDDS_OK) return st;
   }
