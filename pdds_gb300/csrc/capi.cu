@@ -594,12 +594,19 @@ int64_t max_slots(const pdds_ctx* ctx, const pdds_estimate_desc* desc) {
 
 // Table nodes that a path-kernel CTA may stage in shared memory: the largest
 // stencil window that leaves the kernel's 512 threads per SM room, or none
-// where that covers less than half of the knots (a knot whose window is
-// larger reads its nodes through L1).  The line lies at the room because a
-// CTA less per SM costs more than L1's gathers do: tables of 256^2 nodes on
-// 8 x 8 subdomains (room for all windows) 18.4 ms through L1, 17.7 staged;
-// tables of 500^2 (four times the nodes) stay at 24.3 ms.  Returns the bytes.
-size_t lut_stage(const pdds_ctx* ctx, const ProblemDev& P, size_t base_smem, int threads, int* nodes) {
+// where a knot's window is larger (it would read its nodes through the L1 that
+// the others' windows left).  The line lies at the room because a CTA less per
+// SM costs more than L1's gathers do, and at every knot because the ones with
+// the largest windows have the longest paths: where all windows fit (up to
+// 2,900 nodes) staged launches take 0.85 to 1.03 of the time of L1 (333 to
+// 2,205 knots, 100 to 6,000 paths), where 0.59 to 0.97 of the knots' do 0.94
+// to 1.27, and 0.89 to 1.05 at 0.98.  Where sigma and b are the same at every
+// node a staged window saves half of its reads, and half of the knots are
+// enough in launches of eight items per SM or more (the outer loops' tables,
+// 0.98 of the knots: 38.8 -> 24.9 ms; 189 knots, 33 nodes a subdomain: 567
+// items 19.0 ms with, 15.5 without, 2,457 items 26.9 and 29.6).  Returns the
+// bytes.
+size_t lut_stage(const pdds_ctx* ctx, const ProblemDev& P, size_t base_smem, int threads, int n_items, int* nodes) {
   constexpr size_t PER_SM = 228 * 1024, FIXED = 3 * 1024;  // static and reserved shared memory of a CTA
   *nodes = 0;
   const size_t share = PER_SM / (512 / threads);
@@ -617,7 +624,8 @@ size_t lut_stage(const pdds_ctx* ctx, const ProblemDev& P, size_t base_smem, int
   }
   int64_t in = 0;
   for (int v : ctx->mc_host) in += win[L.knot_stencil[v]] <= *nodes;
-  if (2 * in < (int64_t)ctx->mc_host.size()) *nodes = 0;
+  const int64_t all = (int64_t)ctx->mc_host.size();
+  if (in < all && !(ctx->lut_flat && 2 * in >= all && n_items >= 8 * ctx->num_sms)) *nodes = 0;
   return *nodes > 0 ? (size_t)*nodes * 2 * sizeof(float4) + 16 : 0;
 }
 
@@ -798,7 +806,7 @@ pdds_status enqueue_mixed_paths(pdds_ctx* ctx, const pdds_estimate_desc* desc, c
   a.hist_out = ctx->hist.p;
   a.mc_pos = ctx->mc_pos.p;
   a.mc0 = mc0;
-  const size_t smem = base_smem + (mk == PK_LUT ? lut_stage(ctx, P, base_smem, threads, &a.lut_nodes) : 0);
+  const size_t smem = base_smem + (mk == PK_LUT ? lut_stage(ctx, P, base_smem, threads, n_items, &a.lut_nodes) : 0);
   if (smem > MIXED_SMEM_CAP) return hist_refused(ctx);
   int bps = mixed_blocks_per_sm(mk, smem, a.richardson, threads, a.diag != nullptr);
   if (bps < 1) bps = 1;
@@ -1168,6 +1176,7 @@ pdds_status pdds_problem_set_lut(pdds_ctx* ctx, const float* coef, const float* 
   CK(cudaStreamSynchronize(ctx->stream));
   const pdds_status st = build_lut_tex(ctx, coef, nx, ny);
   if (st != PDDS_OK) return st;
+  ctx->lut_flat = false;
   ctx->lut_nx = nx;
   ctx->lut_ny = ny;
   for (int q = 0; q < 4; q++) ctx->lut_bounds[q] = bounds[q];
@@ -1961,6 +1970,7 @@ pdds_status pdds_semilinear_tables(pdds_ctx* ctx, const pdds_semilinear_desc* de
   CK(launch_newton_tables(desc->from_solution ? ctx->ugrid.p : nullptr, G, L.sw[0], L.sw[1], hx, hy, eq,
                           ctx->lut_coef.p, ctx->lut_g.p, s));
   CK(cudaStreamSynchronize(s));
+  ctx->lut_flat = true;
   ctx->lut_nx = G;
   ctx->lut_ny = G;
   ctx->lut_bounds[0] = L.sw[0];

@@ -125,6 +125,7 @@ struct pdds_ctx {
   cudaArray_t lut_arr[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaTextureObject_t lut_tex[4] = {0, 0, 0, 0};
   int lut_nx = 0, lut_ny = 0;
+  bool lut_flat = false;  // sigma and b the same at every node (pdds_semilinear_tables)
   double lut_bounds[4] = {0, 0, 0, 0};
   bool has_layout = false;
   HostLayout L;
