@@ -654,11 +654,17 @@ __global__ void __launch_bounds__(ROWS64_THREADS) k_rows_fp64(const Fp64Args a) 
 
 }  // namespace
 
+// Dynamic shared memory of the largest launch (eight slots' sums and the side
+// knots' coordinates, four sides of 160 knots).  The kernels' limit is always
+// set to this: with the launch's own size, a launch of another context in
+// another thread could lower it in between.
+constexpr int FP64_SMEM_MAX = (FP64_SLOTS + 1) * 4 * 160 * (int)sizeof(double);
+
 template <bool RICH>
 static cudaError_t launch_fp64_t(const Fp64Args& a, int kind, int grid, int threads, size_t smem, cudaStream_t s) {
 #define PDDS_FP64_CASE(KK, GG)                                                                           \
   case KK:                                                                                               \
-    cudaFuncSetAttribute(k_paths_fp64<KK, RICH, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    cudaFuncSetAttribute(k_paths_fp64<KK, RICH, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, FP64_SMEM_MAX); \
     return cudaLaunchKernelEx(&cfg, k_paths_fp64<KK, RICH, GG>, a);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);

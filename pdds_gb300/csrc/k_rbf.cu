@@ -244,9 +244,12 @@ cudaError_t launch_rbf_setup(const DevLayout& L, int max_n, int max_nbins, doubl
   if (max_n > 32 * RBF_SLOTS) return cudaErrorInvalidValue;
   k_psi<<<dim3((max_n * max_n + RBF_THREADS - 1) / RBF_THREADS, L.P), RBF_THREADS, 0, s>>>(L, lu);
   const size_t smem = (size_t)(max_n * max_n) * sizeof(double);
-  cudaFuncSetAttribute(k_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit is always the largest side's: with the launch's own size, a
+  // launch of another context in another thread could lower it in between
+  constexpr int RBF_SMEM_MAX = 32 * RBF_SLOTS * 32 * RBF_SLOTS * (int)sizeof(double);
+  cudaFuncSetAttribute(k_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, RBF_SMEM_MAX);
   k_lu<<<L.P, RBF_THREADS, smem, s>>>(L, lu, piv, uinv, err_flags);
-  cudaFuncSetAttribute(k_lu_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_lu_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, RBF_SMEM_MAX);
   k_lu_inverse<<<dim3((max_n + INV_WARPS - 1) / INV_WARPS, L.P), INV_WARPS * 32, smem, s>>>(L, lu, piv, uinv,
                                                                                            ipsi);
   cudaError_t e = cudaGetLastError();

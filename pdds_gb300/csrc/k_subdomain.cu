@@ -374,6 +374,10 @@ __global__ void k_newton_tables(const double* grid, int G, double x0, double y0,
 }  // namespace
 
 size_t subdomain_smem(int m) { return (size_t)3 * m * m * sizeof(double); }
+// of the largest grid, which the kernels' limit is always set to: with the
+// launch's own size, a launch of another context in another thread could lower
+// it in between
+constexpr int SUB_SMEM_MAX = 3 * 64 * 64 * (int)sizeof(double);
 
 cudaError_t launch_subdomain(const DevLayout& L, const ProblemDev& P, int nsub, int m, int n, const int* edge_knots,
                              const double* u, double* out, double* grid, cudaStream_t s) {
@@ -383,7 +387,7 @@ cudaError_t launch_subdomain(const DevLayout& L, const ProblemDev& P, int nsub, 
   const int G = nsub * (m + 1) + 1;
 #define PDDS_SUB_CASE(KK)                                                                             \
   case KK:                                                                                            \
-    cudaFuncSetAttribute(k_subdomain<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
+    cudaFuncSetAttribute(k_subdomain<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, SUB_SMEM_MAX); \
     k_subdomain<KK><<<nblk, SUB_THREADS, smem, s>>>(L, P, nsub, m, n, edge_knots, u, out, grid, G);   \
     break;
   switch (P.kind) {
@@ -401,7 +405,7 @@ cudaError_t launch_subdomain_lut(const DevLayout& L, const ProblemDev& P, int ns
                                  int* iters, unsigned* err, cudaStream_t s) {
   if (m < 2 || m > 64) return cudaErrorInvalidValue;
   const size_t smem = subdomain_smem(m);
-  cudaFuncSetAttribute(k_subdomain_lut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_subdomain_lut, cudaFuncAttributeMaxDynamicSharedMemorySize, SUB_SMEM_MAX);
   k_subdomain_lut<<<nsub * nsub, SUB_THREADS, smem, s>>>(L, P, nsub, m, n, edge_knots, u, out, work, grid,
                                                          nsub * (m + 1) + 1, max_iter, tol, iters, err);
   return cudaGetLastError();
