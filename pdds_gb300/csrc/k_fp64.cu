@@ -30,10 +30,10 @@
 // seeds), which is why the hand-out may not depend on which warp comes first.
 // With an atomic counter in its place, two runs on the same inputs put 35 %
 // of the further paths into different slots; the exchange that replaces it
-// costs nothing for one knot (742 against 747 us for the whole call) and
-// 1.7 % at 4x4/n11.
-// 4x4/n11, N = 1e4, h = 1e-3: 49.7 -> 25.2 ms; one knot of 5,000 paths
-// 1.02 -> 0.49 ms.
+// costs 1 % at most (one knot 742 against 747 us for the whole call, 4x4/n11
+// 24.84 and 24.80 ms, 12x12/n43 in pairs 3.44 and 3.38 s).
+// 4x4/n11, N = 1e4, h = 1e-3: 49.7 -> 24.8 ms; one knot of 5,000 paths
+// 1.02 -> 0.49 ms; 12x12/n43, 2e4 pairs: 4.64 -> 3.44 s.
 #include <cooperative_groups.h>
 
 #include "dev_common.cuh"
@@ -160,7 +160,8 @@ k_paths_fp64(const Fp64Args a) {
   __shared__ ItemSide64 s_side[4];
   __shared__ double s_rect[4];
   __shared__ int s_item, s_knot, s_nall;
-  __shared__ unsigned s_ends[2][FP64_SLOTS];  // slots: ends in this iteration, and iterations with ends before
+  // slots: ends in this iteration (6 bits), queued exits (8), iterations with ends before
+  __shared__ unsigned s_ends[2][FP64_SLOTS];
   __shared__ double s_h;
   __shared__ double s_red[FP64_THREADS / 32][2];
   __shared__ double s_diag[PDDS_DIAG_N];
@@ -295,8 +296,8 @@ k_paths_fp64(const Fp64Args a) {
       if (d < 0) {
         atomicOr(a.err_flags, ERR_FLAG_EXIT_SIDE);
       } else {
-        // queue the exit: < 32 left over + at most 2 exits per lane and
-        // iteration fit in FP64_QCAP
+        // queue the exit: FP64_QCAP - 64 left over + at most 2 exits per lane
+        // and iteration fit in FP64_QCAP
         const int e = atomicAdd(&s_qn[warp], 1);
         if (idx_ok(e, FP64_QCAP, a.err_flags)) {
           s_qd[warp][e] = d;
@@ -528,8 +529,10 @@ k_paths_fp64(const Fp64Args a) {
       }
       const unsigned fm = __ballot_sync(FULL, fin);
       unsigned take = path_end;
+      int minq = 32;
       if (next < path_end) {
-        const unsigned mine = (unsigned)__popc(fm) | ends << 8;
+        __syncwarp();  // every lane's exits are queued
+        const unsigned mine = (unsigned)__popc(fm) | (unsigned)s_qn[warp] << 6 | ends << 14;
         unsigned* slots = s_ends[phase];
         if (a.spread) {
           if (lane < groups) *cluster.map_shared_rank(slots + slot, lane) = mine;
@@ -538,12 +541,16 @@ k_paths_fp64(const Fp64Args a) {
           if (lane == 0) slots[slot] = mine;
           __syncthreads();
         }
-        const unsigned other = lane < FP64_SLOTS ? slots[lane] : 0u, n = other & 0xffu;
-        const bool first = other >> 8 < ends || (other >> 8 == ends && lane > slot);
+        const unsigned other = lane < FP64_SLOTS ? slots[lane] : 0u, n = other & 0x3fu, before = other >> 14;
+        const bool first = before < ends || (before == ends && lane > slot);
         take = next + __reduce_add_sync(FULL, first ? n : 0u) + (unsigned)__popc(fm & lt);
         next += __reduce_add_sync(FULL, n);
-        ends += fm != 0u;
+        ends = min(ends + (fm != 0u ? 1u : 0u), 0x3ffffu);
         phase ^= 1u;
+        // warps in step add their exits together: one that did it alone would
+        // hold up the others (for as long as seven iterations with 127 side
+        // knots: 12x12/n43 5.5 s, together 3.4)
+        minq = __reduce_max_sync(FULL, other >> 6 & 0xffu) > FP64_QCAP - 64 ? 1 : FP64_QCAP + 1;
       }
       if (fin) {
         path = take;
@@ -556,7 +563,7 @@ k_paths_fp64(const Fp64Args a) {
           m = 0;
         }
       }
-      flush(32);
+      flush(minq);
     }
     flush(1);
     __syncthreads();

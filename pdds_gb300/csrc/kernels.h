@@ -16,7 +16,7 @@ constexpr int MIXED_MAX_THREADS = 256;
 inline int mixed_threads(int n_mc) { return n_mc >= 8192 ? 128 : 256; }
 constexpr int FP64_SLOTS = 8;      // warps that share a block of paths in the FP64 kernel
 constexpr int FP64_THREADS = 32 * FP64_SLOTS;  // at most (a CTA may take fewer slots)
-constexpr int FP64_QCAP = 96;  // exits queued per warp in the FP64 kernel
+constexpr int FP64_QCAP = 160;  // exits queued per warp in the FP64 kernel
 constexpr unsigned ERR_FLAG_STEP_LIMIT = 1u;
 constexpr unsigned ERR_FLAG_EXIT_SIDE = 2u;
 constexpr unsigned ERR_FLAG_SINGULAR = 4u;
