@@ -16,8 +16,11 @@ plain FP64 GPU form are measured beside it.
          context with the layout built on the host and uploaded, estimation,
          solve, and G/B/u copied back to host, every step (after the same
          warm-up steps as the device-timed step)
-  roofline  FP32 issue-slot roof of the path kernel (the path is issue-bound:
-         it reads a few MB of stencil tables and no large arrays)
+  roofline  counted operations of the paths against the FP32 issue-slot roof
+         (the path is issue-bound: its one large array is the exit histograms,
+         written by the path kernel and read by the contraction), over the
+         interval of the path kernel, the contraction and what is left of the
+         factorisation and tables, which run beside the paths
   cpu_baseline  the CPU restatement of the reference (OpenMP paths, serial
          O(n_s^2) reduction), on a bounded sample of knots of the same workload
 
@@ -44,7 +47,10 @@ if ROOT not in sys.path:
 METRIC = "path-steps/s & interface solves/s at RMSE<=2e-3, mixed+batched vs plain FP64"
 
 # Algorithmic thread-instruction counts (fixed before tuning, counted from the
-# algorithm, not from the compiler): one Euler-Maruyama step = half a
+# algorithm in its plain form, not from the compiler; a count, not a lower
+# bound: the kernel's exit test is two comparisons and some instructions do two
+# operations, so by the counters it takes 74 % of the issue slots with 23.8 of
+# 32 lanes active where this count gives 0.71 of the roof): one Euler-Maruyama step = half a
 # Philox-4x32-10 call (10 rounds of 2 wide multiplies and 2 three-way XORs,
 # 40 INT) + Box-Muller (2 converts, log, sqrt, sin, cos, 4 FP32: 10) +
 # Poisson coefficients (sin/cos of pi x and pi y, source, gradient: 14) +
@@ -56,11 +62,15 @@ METRIC = "path-steps/s & interface solves/s at RMSE<=2e-3, mixed+batched vs plai
 W_STEP = 94
 W_EXIT = 42
 
-# DRAM bytes (read + write) of one k_paths_mixed launch, from one ncu capture
-# of the same workload (dram__bytes_read.sum + dram__bytes_write.sum); the
-# captures and their commands are summarised under profiles/.
+# DRAM bytes (read + write) of one k_paths_mixed and one k_contract launch, from
+# one ncu capture of the same workload (dram__bytes_read.sum +
+# dram__bytes_write.sum, caches as the launches leave them); the captures and
+# their commands are summarised under profiles/.
 PATH_KERNEL_DRAM_BYTES = {
-    "poisson_12x12_n43": 35_996_672,
+    "poisson_12x12_n43": 162_753_024,
+}
+CONTRACT_DRAM_BYTES = {
+    "poisson_12x12_n43": 260_904_704,
 }
 
 
@@ -765,7 +775,7 @@ def main():
             cpu = {"value": None, "unit": "path-steps/s", "cores": os.cpu_count(), "kind": "port",
                    "sample": f"failed: {exc}"}
 
-    # issue-slot roofline of the path kernel
+    # issue-slot roofline of the paths
     sm_count = torch.cuda.get_device_properties(local).multi_processor_count
     f_mhz = clk.get("sm_mhz") or 1920.0
     peak = sm_count * 4 * 32 * f_mhz * 1e6  # thread-instructions per second
@@ -775,7 +785,9 @@ def main():
     roof = {"bound": "issue", "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "Ginst/s",
             "frac": achieved / peak, "traffic": PATH_KERNEL_DRAM_BYTES.get(workload["name"]),
             "peak_source": f"{sm_count} SMs x 128 issue lanes x median SM clock {f_mhz:.0f} MHz under load",
-            "kernel": "k_paths_mixed", "kernel_ms_per_launch": 1000 * t_paths / args.steps}
+            "kernel": "k_paths_mixed", "kernel_ms_per_launch": 1000 * t_paths / args.steps,
+            "interval": "k_paths_mixed, k_contract and the end of the RBF set-up beside them",
+            "traffic_contraction": CONTRACT_DRAM_BYTES.get(workload["name"])}
 
     line = {
         "metric": METRIC, "value": value, "unit": "path-steps/s", "n_gpus": world, "steps": args.steps,
