@@ -34,8 +34,12 @@ int batch_waves(const pdds_ctx* ctx, const pdds_batch_run_desc* d) {
 // in it (10 groups) 10 ms.  Not for many systems at once, which fill the
 // chip: one takes a third (237 rows) to a ninth (19,005 rows) of the cluster
 // kernel's time, but one follows the other, and the cluster kernel runs
-// num_sms / cluster at a time.  The classical form and systems that do not
-// fit keep the cluster.
+// num_sms / cluster at a time.  In batches of n equal instances, one group,
+// one after the other is the faster up to n = 3 (237 and 5,181 rows), 4 (741
+// and 2,205 rows) and 5 (7,821 rows), and at all n to 10 for 10,989 and 19,005
+// rows; on the wrong side of the line the rule costs 14 % up to 5,181 rows and
+// 25 % at most (8 systems of 10,989 rows, 33.7 ms instead of 27.0).  The
+// classical form and systems that do not fit keep the cluster.
 int tail_systems(int max_rows) { return 3 + max_rows / 3000; }
 const std::vector<ResidentPlan>& batch_tail(pdds_ctx* ctx, const pdds_batch_run_desc* d, int cluster, int i0, int m) {
   pdds_ctx::BatchTail& t = ctx->batch_tail;

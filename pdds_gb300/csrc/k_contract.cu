@@ -17,9 +17,9 @@
 // instruction forms the products of two items.  The stages come by
 // asynchronous copies, two ahead (a shape's CT_BINS x n weights are
 // contiguous).  Loads into registers, one ahead, took 0.63 ms at 12x12/n43,
-// the copies 0.52, two products per instruction 0.46.  Path kernel and
-// contraction: 24.9 -> 22.5 ms there; 237 knots 0.433 -> 0.402 ms; 741 knots
-// with variances 3.50 -> 3.42.
+// the copies 0.52, two products per instruction 0.46, the third float of the
+// sums 0.51.  Path kernel and contraction: 24.9 -> 22.6 ms there; 237 knots
+// 0.433 -> 0.404 ms; 741 knots with variances 3.50 -> 3.43.
 //
 // Rounding is that of the loop it replaces: FP32 sums of 64 products in the
 // same order for each item, added to more than FP64 accuracy in three floats

@@ -30,10 +30,10 @@
 // seeds), which is why the hand-out may not depend on which warp comes first.
 // With an atomic counter in its place, two runs on the same inputs put 35 %
 // of the further paths into different slots; the exchange that replaces it
-// costs 1 % at most (one knot 742 against 747 us for the whole call, 4x4/n11
-// 24.84 and 24.80 ms, 12x12/n43 in pairs 3.44 and 3.38 s).
+// costs up to 5 % (one knot 742 against 747 us for the whole call, 4x4/n11
+// 24.84 and 24.80 ms, 12x12/n43 in pairs 3.44 to 3.59 and 3.38 to 3.41 s).
 // 4x4/n11, N = 1e4, h = 1e-3: 49.7 -> 24.8 ms; one knot of 5,000 paths
-// 1.02 -> 0.49 ms; 12x12/n43, 2e4 pairs: 4.64 -> 3.44 s.
+// 1.02 -> 0.49 ms; 12x12/n43, 2e4 pairs: 4.64 -> 3.5 s.
 #include <cooperative_groups.h>
 
 #include "dev_common.cuh"

@@ -810,7 +810,9 @@ k_paths_mixed(const MixedArgs a) {
     // four-operation exit test, which went at the same time): 12x12/n43
     // 27.3 -> 25.0 ms, the circle at h = 2e-5 (270 rounds per pair) 341 ->
     // 290 ms; GAP 8, 14, 22, 32 and 36 measured 27.4, 26.7, 25.2, 25.0 and
-    // 25.0 ms on the former.  A round of
+    // 25.0 ms on the former; without pairs GAP 12, 24, 48 and 96 measured 430,
+    // 413, 394 and 393 us (4x4/n11), 2.22, 2.07, 2.03 and 2.05 ms (8x8/n21),
+    // 3.10, 3.10, 3.02 and 3.15 ms (741 knots with variances).  A round of
     // the table-served kinds is bound by its table reads, which idle lanes
     // do not shorten (groups measured 1-2 % slower there): they look after
     // every round.

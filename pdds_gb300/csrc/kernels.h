@@ -11,8 +11,11 @@ namespace pdds {
 
 constexpr int MIXED_MAX_THREADS = 256;
 // Block size of the MIXED path kernel: 128-thread CTAs (8 per SM) for large
-// layouts, where they were faster (12x12/n43: 27.7 against 28.2 ms), 256
-// (4 per SM) below 8192 Monte Carlo knots, where 128 measured 6-17 % slower.
+// layouts, 256 (4 per SM) below 8192 Monte Carlo knots, except for short work
+// items and long continuations (short_items and adaptive_continue in capi.cu).
+// 128 against 256, 20,000 paths: 10,989 knots in pairs 22.5 and 22.8 ms, with
+// variances (whose histograms leave 128-thread CTAs fewer lanes per SM) 9.1 and
+// 7.4; 3,325 knots in pairs 6.9 and 6.6, with variances 2.5 and 2.2.
 inline int mixed_threads(int n_mc) { return n_mc >= 8192 ? 128 : 256; }
 constexpr int FP64_SLOTS = 8;      // warps that share a block of paths in the FP64 kernel
 constexpr int FP64_THREADS = 32 * FP64_SLOTS;  // at most (a CTA may take fewer slots)
