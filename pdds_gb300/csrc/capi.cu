@@ -1741,7 +1741,11 @@ pdds_status pdds_autotune(pdds_ctx* ctx, const pdds_estimate_desc* desc, int32_t
       ctx->force_grid_frac = frac;
       CK(cudaEventRecord(ctx->ev0, s));
       int nl = 0;
-      pdds_status e = enqueue_mixed_paths(ctx, &d, P, 1, ppc, &nl, &items);
+      // with the set-up beside the paths where an estimate has it there: a long
+      // item that it delays ends the launch late (circle, 2,128 knots, 20,000
+      // pairs; the shape chosen without it 12.8 ms, with it 10.1, untuned 10.0)
+      pdds_status e = ns == (int)mc.size() ? enqueue_prefix(ctx, &d, P, false, &nl) : PDDS_OK;
+      if (e == PDDS_OK) e = enqueue_mixed_paths(ctx, &d, P, 1, ppc, &nl, &items);
       ctx->force_bps = 0;
       ctx->force_grid_frac = 0.0;
       if (e != PDDS_OK) return e;
